@@ -50,7 +50,7 @@ typedef SieveGeom<8192, 256> SieveNarrow;
 #endif
 constexpr int kTestThreads = WW_TEST_THREADS;
 #ifndef WW_TEST_MINB
-#define WW_TEST_MINB 1  // minimum resident CTAs per SM asked of the test kernels
+#define WW_TEST_MINB 4  // resident CTAs per SM asked of the test kernels: 64 registers, 32 warps
 #endif
 
 struct HitOut {

@@ -1,0 +1,261 @@
+// ww_ladder.cuh -- the two-digit arithmetic of the test ladders, with the
+// corrections it does not need left out.
+//
+// A residue is X = x0 + p*x1 in Montgomery form, R = 2^64, as in
+// ww_arith.cuh, but only x0 is canonical: x1 is any representative in
+// [0, 2p) that fits 64 bits.  With x0 < p the low digit of a product needs
+// one conditional addition of p, as there; its high digit
+//     T = (C + u + k1) / 2^64 - v - borrow,   C = 2 x0 x1 (or x0 y1 + x1 y0)
+// lies in [-p, 2p), and t = T >> 64 is -1, 0 or 1: T - t p fits 64 bits again
+// and is below 2p, so one three-way correction replaces the two of the
+// canonical form.  The constant of a ladder step (k0 + p k1 = c R^2 mod p^2)
+// is added before the reduction, where it costs two additions and no
+// correction.
+//
+// What bounds it (B200, cycles of one of an SM's four schedulers): a 32x32->64
+// multiply holds the multiply pipe for 4 cycles and the ALU side for 2.3,
+// any other integer instruction holds its pipe for 2, and the compiler
+// spreads moves and carries over both, so the time is about 3.15 cycles a
+// wide multiply and one for every other instruction, of which 87 % is
+// reached; occupancy (48 to 80 registers) moves it by 1 %.  A ladder step was
+// 319 instructions (54 wide multiplies) and is 235 (59) now.  Products are
+// unsigned __int128 ones: a 64x64->128 product is then 7.4 instructions and 16
+// cycles of the multiply pipe, against 11.5 and 24 for `a * b` beside
+// `__umul64hi(a, b)`, which share nothing.  Both tests over 2^24 primes of
+// [2^62, 2^64): 12.33 ms with canonical digits, a pair of squarings and
+// doublings bit by bit, 10.78 ms in this form (1 360 and 1 557 M primes/s).
+#pragma once
+
+#include "ww_arith.cuh"
+
+namespace ww {
+
+typedef unsigned __int128 u128;
+
+struct LzMod {
+    u64 p, q;      // q = p^-1 mod 2^64
+    u32 npl, nph;  // -p = npl + 2^32 nph mod 2^64, npl signed
+};
+
+WW_HD LzMod lz_mod(u64 p, u64 q) {
+    LzMod m;
+    m.p = p;
+    m.q = q;
+    const u64 n = 0 - p;
+    m.npl = (u32)n;
+    m.nph = (u32)(n >> 32) + (m.npl >> 31);
+    return m;
+}
+
+// r - t p mod 2^64 for t in {-1, 0, 1} (a word, -1 as 2^32 - 1): a signed
+// wide multiply-add and a multiply-add, two instructions (by two selects and
+// a predicated add: 1 433 against 1 504 M primes/s).
+WW_HD u64 lz_fix(u64 r, u32 t, const LzMod &m) {
+#if defined(__CUDA_ARCH__)
+    u64 o;
+    asm("{\n\t.reg .u32 l, h;\n\t"
+        "mad.wide.s32 %0, %1, %2, %3;\n\t"
+        "mov.b64 {l, h}, %0;\n\t"
+        "mad.lo.u32 h, %1, %4, h;\n\t"
+        "mov.b64 %0, {l, h};\n\t}"
+        : "=l"(o) : "r"(t), "r"(m.npl), "l"(r), "r"(m.nph));
+    return o;
+#else
+    return r - (u64)(long long)(int)t * m.p;
+#endif
+}
+// r + (neg ? p : 0) for the mask neg (0 or 2^32 - 1), on the ALU: 1 504 M
+// primes/s, against 1 492 M with the "& p" as two multiplies by the mask and
+// 1 467 M as lz_fix.
+WW_HD u64 lz_addp(u64 r, u32 neg, const LzMod &m) {
+#if defined(__CUDA_ARCH__)
+    u64 t;
+    asm("{\n\t.reg .u32 a0, a1, r0, r1;\n\t"
+        "mov.b64 {a0, a1}, %2;\n\t"
+        "mov.b64 {r0, r1}, %3;\n\t"
+        "and.b32 a0, a0, %1;\n\t"
+        "and.b32 a1, a1, %1;\n\t"
+        "add.cc.u32 r0, r0, a0;\n\t"
+        "addc.u32 r1, r1, a1;\n\t"
+        "mov.b64 %0, {r0, r1};\n\t}"
+        : "=l"(t) : "r"(neg), "l"(m.p), "l"(r));
+    return t;
+#else
+    return neg ? r + m.p : r;
+#endif
+}
+
+// a - b mod 2^64 and the borrow as a mask
+WW_HD u64 lz_sub(u64 a, u64 b, u32 &neg) {
+#if defined(__CUDA_ARCH__)
+    u64 r;
+    asm("sub.cc.u64 %0, %2, %3;\n\t"
+        "subc.u32 %1, 0, 0;"
+        : "=&l"(r), "=r"(neg) : "l"(a), "l"(b));
+    return r;
+#else
+    neg = a < b ? ~0u : 0u;
+    return a - b;
+#endif
+}
+
+// a^2 from three 32x32 products: a0^2 + 2^64 a1^2 and a0 a1 shifted in by 33
+// bits.  One wide multiply fewer than a product of a by itself.
+WW_HD u128 lz_square(u64 a) {
+#if defined(__CUDA_ARCH__)
+    u64 lo, hi;
+    asm("{\n\t.reg .u64 e, f, o;\n\t.reg .u32 r0, r1, r2, r3, x, y, z;\n\t"
+        "mul.wide.u32 e, %2, %2;\n\t"
+        "mul.wide.u32 o, %2, %3;\n\t"
+        "mul.wide.u32 f, %3, %3;\n\t"
+        "mov.b64 {r0, r1}, e;\n\t"
+        "mov.b64 {r2, r3}, f;\n\t"
+        "mov.b64 {x, y}, o;\n\t"
+        "shf.l.clamp.b32 z, x, y, 1;\n\t"
+        "shl.b32 x, x, 1;\n\t"
+        "shr.u32 y, y, 31;\n\t"
+        "add.cc.u32 r1, r1, x;\n\t"
+        "addc.cc.u32 r2, r2, z;\n\t"
+        "addc.u32 r3, r3, y;\n\t"
+        "mov.b64 %0, {r0, r1};\n\t"
+        "mov.b64 %1, {r2, r3};\n\t}"
+        : "=l"(lo), "=l"(hi) : "r"((u32)a), "r"((u32)(a >> 32)));
+    return ((u128)hi << 64) | lo;
+#else
+    return (u128)a * a;
+#endif
+}
+
+// Low digit of T / R for T < p 2^64: the digit, u = T q mod 2^64 and the
+// borrow mask that the high digit takes over.
+WW_HD u64 lz_low(u128 T, const LzMod &m, u64 &u, u32 &neg) {
+    u = (u64)T * m.q;
+    const u64 r = lz_sub((u64)(T >> 64), mul_hi(u, m.p), neg);
+    return lz_addp(r, neg, m);
+}
+
+// High digit from the sum (k:h:s), k signed: ((k:h) - hi(s q p)) in [-p, 2p).
+WW_HD u64 lz_high(u64 s, u64 h, u32 k, const LzMod &m) {
+    const u64 v = mul_hi(s * m.q, m.p);
+#if defined(__CUDA_ARCH__)
+    u64 r;
+    u32 t;
+    asm("sub.cc.u64 %0, %2, %3;\n\t"
+        "subc.u32 %1, %4, 0;"
+        : "=&l"(r), "=r"(t) : "l"(h), "l"(v), "r"(k));
+    return lz_fix(r, t, m);
+#else
+    const __int128 T = (((__int128)(int)k) << 64) + h - v;
+    return (u64)T - (u64)(long long)(T >> 64) * m.p;
+#endif
+}
+
+// (k:h:s) = a + b + u + k1 + 2^64 neg, neg a borrow mask (0 or -1).
+WW_HD void lz_sum(u128 a, u128 b, u64 u, u64 k1, u32 neg, u64 &s, u64 &h, u32 &k) {
+#if defined(__CUDA_ARCH__)
+    u64 neg2;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(neg2) : "r"(neg));
+    asm("add.cc.u64 %0, %3, %5;\n\t"
+        "addc.cc.u64 %1, %4, %6;\n\t"
+        "addc.u32 %2, 0, %9;\n\t"
+        "add.cc.u64 %0, %0, %7;\n\t"
+        "addc.cc.u64 %1, %1, 0;\n\t"
+        "addc.u32 %2, %2, 0;\n\t"
+        "add.cc.u64 %0, %0, %8;\n\t"
+        "addc.cc.u64 %1, %1, %10;\n\t"
+        "addc.u32 %2, %2, 0;"
+        : "=&l"(s), "=&l"(h), "=&r"(k)
+        : "l"((u64)a), "l"((u64)(a >> 64)), "l"((u64)b), "l"((u64)(b >> 64)), "l"(u), "l"(k1), "r"(neg), "l"(neg2));
+#else
+    u128 t = a + b;
+    k = t < a;
+    t += u;
+    k += t < u;
+    t += k1;
+    k += t < k1;
+    s = (u64)t;
+    h = (u64)(t >> 64);
+    if (neg) k -= h-- == 0;
+#endif
+}
+// the same without k1
+WW_HD void lz_sum(u128 a, u128 b, u64 u, u32 neg, u64 &s, u64 &h, u32 &k) {
+#if defined(__CUDA_ARCH__)
+    u64 neg2;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(neg2) : "r"(neg));
+    asm("add.cc.u64 %0, %3, %5;\n\t"
+        "addc.cc.u64 %1, %4, %6;\n\t"
+        "addc.u32 %2, 0, %8;\n\t"
+        "add.cc.u64 %0, %0, %7;\n\t"
+        "addc.cc.u64 %1, %1, %9;\n\t"
+        "addc.u32 %2, %2, 0;"
+        : "=&l"(s), "=&l"(h), "=&r"(k)
+        : "l"((u64)a), "l"((u64)(a >> 64)), "l"((u64)b), "l"((u64)(b >> 64)), "l"(u), "r"(neg), "l"(neg2));
+#else
+    lz_sum(a, b, u, 0, neg, s, h, k);
+#endif
+}
+
+// X^2 / R
+WW_HD D2 lz_sqr(D2 x, const LzMod &m) {
+    u64 u, s, h;
+    u32 neg, k;
+    D2 r;
+    r.d0 = lz_low(lz_square(x.d0), m, u, neg);
+    const u128 c = (u128)x.d0 * x.d1;
+    lz_sum(c, c, u, neg, s, h, k);
+    r.d1 = lz_high(s, h, k, m);
+    return r;
+}
+// (X^2 + K) / R, K canonical
+WW_HD D2 lz_sqr_add(D2 x, D2 kk, const LzMod &m) {
+    u64 u, s, h;
+    u32 neg, k;
+    D2 r;
+    r.d0 = lz_low(lz_square(x.d0) + kk.d0, m, u, neg);
+    const u128 c = (u128)x.d0 * x.d1;
+    lz_sum(c, c, u, kk.d1, neg, s, h, k);
+    r.d1 = lz_high(s, h, k, m);
+    return r;
+}
+// (X Y + K) / R, K canonical
+WW_HD D2 lz_mul_add(D2 x, D2 y, D2 kk, const LzMod &m) {
+    u64 u, s, h;
+    u32 neg, k;
+    D2 r;
+    r.d0 = lz_low((u128)x.d0 * y.d0 + kk.d0, m, u, neg);
+    lz_sum((u128)x.d0 * y.d1, (u128)x.d1 * y.d0, u, kk.d1, neg, s, h, k);
+    r.d1 = lz_high(s, h, k, m);
+    return r;
+}
+
+// X 2^(d - 32) for 0 <= d < 32: each digit shifted left by d and reduced by
+// one 32-bit Montgomery step.
+WW_HD D2 lz_shift(D2 x, u32 d, const LzMod &m) {
+    const u32 q0 = (u32)m.q, p0 = (u32)m.p, p1 = (u32)(m.p >> 32);
+    D2 r;
+    u32 neg, neg1;
+    // low digit: T = x0 2^d, (T - w p) / 2^32 with w = T q mod 2^32
+    const u64 h0 = x.d0 >> (32 - d);  // T >> 32 (d = 0: x0 >> 32)
+    const u32 w = ((u32)x.d0 << d) * q0;
+    const u64 v = (u64)w * p1 + (((u64)w * p0) >> 32);
+    const u64 r0 = lz_sub(h0, v, neg);
+    r.d0 = lz_addp(r0, neg, m);
+    // high digit: x1 2^d + w the same way, less the borrow
+    const u32 c0 = (u32)x.d1 << d;
+    const u32 s0 = c0 + w;
+    const u64 h1 = (x.d1 >> (32 - d)) + (u64)(s0 < w);
+    const u32 w1 = s0 * q0;
+    const u64 v1 = (u64)w1 * p1 + (((u64)w1 * p0) >> 32) + (u64)(neg & 1u);
+    const u64 r1 = lz_sub(h1, v1, neg1);
+    r.d1 = lz_addp(r1, neg1, m);
+    return r;
+}
+
+// x1 < 2p made canonical
+WW_HD D2 lz_canonical(D2 x, u64 p) {
+    if (x.d1 >= p) x.d1 -= p;
+    return x;
+}
+
+}  // namespace ww

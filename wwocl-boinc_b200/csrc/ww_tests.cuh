@@ -1,14 +1,16 @@
 // ww_tests.cuh -- the Wieferich and Wall-Sun-Sun tests of one prime, and the
 // reference's hit classification.
 //
-// The mod p^2 arithmetic is a policy: Arith64 uses 64-bit C products
-// (ww_arith.cuh), Arith32 explicit 32-bit PTX carry chains and ArithWide
-// 32x32+64 wide products (ww_chain.cuh).  All produce the same canonical
-// digits; kernels and the host self-test use WW_ARITH.
+// The ladders run on the two-digit arithmetic of ww_ladder.cuh.  Arith64
+// (64-bit C products, ww_arith.cuh), Arith32 (explicit 32-bit PTX carry
+// chains) and ArithWide (32x32+64 wide products, ww_chain.cuh) are the
+// canonical forms that the operand-level checks compare; WW_ARITH also sets
+// the PRP test's form.
 #pragma once
 
 #include "ww_arith.cuh"
 #include "ww_chain.cuh"
+#include "ww_ladder.cuh"
 
 namespace ww {
 
@@ -75,254 +77,187 @@ WW_HD D2 sel(bool c, D2 a, D2 b) {
     return r;
 }
 
-// Lucas numbers V_k (P = 1, Q = -1: V_0 = 2, V_1 = 1) for 32 <= k <= 64, all
-// below 2^45: the Lucas ladder's state after the top six bits of its index.
-#define WW_LUCAS_32_64                                                                                \
-    4870847ull, 7881196ull, 12752043ull, 20633239ull, 33385282ull, 54018521ull, 87403803ull,        \
-        141422324ull, 228826127ull, 370248451ull, 599074578ull, 969323029ull, 1568397607ull,        \
-        2537720636ull, 4106118243ull, 6643838879ull, 10749957122ull, 17393796001ull, 28143753123ull, \
-        45537549124ull, 73681302247ull, 119218851371ull, 192900153618ull, 312119004989ull,          \
-        505019158607ull, 817138163596ull, 1322157322203ull, 2139295485799ull, 3461452808002ull,     \
-        5600748293801ull, 9062201101803ull, 14662949395604ull, 23725150497407ull
+// W_k = V_2k, the Lucas numbers of even index (P = 3, Q = 1), for 0 <= k <= 33,
+// all below 2^46: the ladder's state after the top bits of its index.
+#define WW_LUCAS_EVEN                                                                                       \
+    2ull, 3ull, 7ull, 18ull, 47ull, 123ull, 322ull, 843ull, 2207ull, 5778ull, 15127ull, 39603ull,           \
+        103682ull, 271443ull, 710647ull, 1860498ull, 4870847ull, 12752043ull, 33385282ull, 87403803ull,     \
+        228826127ull, 599074578ull, 1568397607ull, 4106118243ull, 10749957122ull, 28143753123ull,           \
+        73681302247ull, 192900153618ull, 505019158607ull, 1322157322203ull, 3461452808002ull,               \
+        9062201101803ull, 23725150497407ull, 62113250390418ull
 #if defined(__CUDACC__)
-static __device__ const u64 g_lucas_32_64[33] = {WW_LUCAS_32_64};
+static __device__ const u64 g_lucas_even[34] = {WW_LUCAS_EVEN};
 #endif
-static const u64 h_lucas_32_64[33] = {WW_LUCAS_32_64};
+static const u64 h_lucas_even[34] = {WW_LUCAS_EVEN};
 
-WW_HD u64 lucas_small(u32 k) {  // 32 <= k <= 64
+WW_HD u64 lucas_even(u32 k) {  // k <= 33
 #if defined(__CUDA_ARCH__)
-    return __ldg(&g_lucas_32_64[k - 32]);
+    return __ldg(&g_lucas_even[k]);
 #else
-    return h_lucas_32_64[k - 32];
+    return h_lucas_even[k];
 #endif
 }
 
-// Where the ladders start.  Each takes the bits of its exponent below its
-// start bit in the loop and begins from the value of the bits above it:
-//   Lucas: i0 = top_bit(n) - 6 for n = p - (p|5); k0 = n >> (i0 + 1) is the
-//          top six bits of n (32 <= k0 < 64), so the pair (V_k0, V_k0+1)
-//          comes from lucas_small;
-//   Wieferich: iw = top_bit(e) - 5 for e = (p-1)/2; e0 = e >> (iw + 1) is the
-//          top five bits of e (16 <= e0 < 32), so the start is 2^e0.
-// e has one bit fewer than n, so iw = i0 (two fewer when p + 1 is a power of
-// two, and then the first loop step is the Lucas ladder's alone).  m2_small
-// turns each start into Montgomery form with two exact reductions: six
-// reductions of about 25 instructions replace the first five ladder steps
-// (ten squarings) and four Wieferich squarings.
-struct LadderStart {
-    int i0, iw;
-    bool odd;  // parity of the Lucas index k0
-    D2 a, b, w;
-    double rp;  // 1 / (double)p
-};
-
-WW_HD LadderStart ladder_start(u64 p, u64 n, D2 one) {
-    LadderStart st;
-    const u64 e = p >> 1;
-    st.i0 = top_bit(n) - 6;
-    st.iw = top_bit(e) - 5;
-    const u32 k0 = (u32)(n >> (st.i0 + 1));
-    const u32 e0 = (u32)(e >> (st.iw + 1));
-    const double rp = 1.0 / (double)p;
-    st.rp = rp;
-    st.odd = k0 & 1u;
-    st.a = m2_small(lucas_small(k0), one, p, rp);
-    st.b = m2_small(lucas_small(k0 + 1), one, p, rp);
-    st.w = m2_small(1ull << e0, one, p, rp);
-    return st;
+// The two exponents have the same length to within a bit: (p-1)/2 for the
+// Wieferich powering of 2, and j = (p - (p|5))/2 for the Lucas ladder, since
+// F_2j comes from W_j and W_j+1.  Both ladders take the same number of steps,
+// and so do all lanes of a warp: the warp's longest j less five bits.  What
+// lies above the steps' bits is at most 5 bits of the start (31, or 32 for a
+// j of 2^k), fewer for a lane whose p is shorter.
+WW_HD u64 lucas_index(u64 p) {
+    const u32 pm5 = (u32)(p % 5);
+    return ((pm5 == 2 || pm5 == 3) ? p + 1 : p - 1) >> 1;
+}
+// every lane of the warp calls it
+WW_HD int ladder_steps(u64 j) {
+    int top = j ? top_bit(j) : 0;
+#if defined(__CUDA_ARCH__)
+    top = (int)__reduce_max_sync(0xffffffffu, (unsigned)top);
+#endif
+    return top > 4 ? top - 4 : 0;
 }
 
-// 2^((p-1)/2) mod p^2 as canonical digits: left-to-right powering of 2, a
-// squaring per exponent bit and a doubling where the bit is set
-// (wieferich.cl:219-245), from 2^e0 for the top five bits e0 of the exponent.
-template <class A>
-WW_HD D2 wieferich_digits_t(u64 p, u64 q, D2 one) {
-    const A ar(p, q);
-    const u64 e = p >> 1;
-    const int i0 = top_bit(e) - 5;
-    const double rp = 1.0 / (double)p;
-    D2 a = m2_small(1ull << (u32)(e >> (i0 + 1)), one, p, rp);
-    u64 eb = e << (63 - i0);  // bit i of e at bit 63 in step i
-    for (int i = i0; i >= 0; --i) {
-        a = ar.sqr(a);
-#if defined(WW_W_WINDOW)
-        if (((i0 - i) & 3) == 3) a = m2_mul_pow2(a, (u32)(e >> i) & 15u, p, rp);
-#else
-        a = sel((long long)eb < 0, m2_dbl(a, p), a);
-#endif
-        eb <<= 1;
+// Wieferich: 2^e by left-to-right squaring; the bits of e are multiplied in
+// five at a time as 2^(d-32), 0 <= d < 32 (lz_shift: two one-word Montgomery
+// steps, 6 instructions a bit where a conditional doubling of two digits
+// takes 18).  With f = e + sum of 32^(w+1) over the windows w, e is the start
+// f >> steps (below 48) times 2^steps plus the sum of (d_w - 32) 32^w.
+constexpr int kWBits = 5;
+WW_HD u64 wieferich_windows(u64 e, int steps) {
+    // 32 + 32^2 + ... for ceil(steps / 5) windows: 32 (32^n - 1) / 31
+    const int n = (steps + kWBits - 1) / kWBits;
+    const u64 ones = 0x0842108421084210ull << 1;  // bits 5, 10, ..., 60
+    return e + (ones & ((2ull << (kWBits * n)) - 1));
+}
+
+// The digit of the window at bit pos, below bit i (the top window is short).
+WW_HD u32 window_digit(u64 f, int pos, int i) { return (u32)(f >> pos) & ((1u << (i - pos)) - 1u); }
+
+// L R mod p^2 as canonical digits for L < 2^48.  For p >= 2^62 the quotient
+// of L 2^64 by p is below 2^50 and mod_est's estimate within 2^-1 of it (three
+// roundings of 2^-53 and those of (double)p), so its correction by one is
+// still enough; and it is the high digit as it stands: one reduction, where
+// m2_small needs two and the products with the digits of R.
+WW_HD D2 small_start(u64 L, D2 one, u64 p, double rp) {
+    if (p >> 62) {
+        D2 r;
+        r.d0 = mod_est(L, 0, p, rp, r.d1);
+        return r;
     }
-#if defined(WW_W_WINDOW)
-    const int rest = (i0 + 1) & 3;
-    if (rest) a = m2_mul_pow2(a, (u32)e & ((1u << rest) - 1u), p, rp);
-#endif
-    return ar.redc(a);
+    return m2_small(L, one, p, rp);
 }
 
-// One step of the Lucas ladder kept as (e, o): for the pair of indices
-// (k, k+1), e is V at the even one and o is V at the odd one up to sign.
-// Since V_2m = V_m^2 - 2(-1)^m, x = e^2 - 2 and y = o^2 + 2 are V at twice
-// the even and twice the odd index, whatever the parity of k, and their
-// difference is V_2k+1 up to sign (y - x = +V_2k+1 for k even, -V_2k+1 for k
-// odd), which the next squaring does not see.  The new pair is (2k, 2k+1)
-// for bit 0 and (2k+1, 2k+2) for bit 1; its even index is 2k or 2k+2, so e
-// becomes x or y by the bit and the parity of k.  Against a ladder on
-// (V_k, V_k+1) this saves the selection of the constant -2(-1)^k and one of
-// the two pair selections.  two and mtwo: 2 and -2 in Montgomery form.
-template <class A>
-WW_HD void eo_step(const A &ar, D2 &e, D2 &o, bool &kodd, bool bit, D2 two, D2 mtwo, u64 p) {
-    const D2 x = m2_sub(ar.sqr(e), two, p);   // V_2k (k even) or V_2k+2 (k odd)
-    const D2 y = m2_sub(ar.sqr(o), mtwo, p);  // the other of the two
-    o = m2_sub(y, x, p);
-    e = sel(bit != kodd, y, x);
+struct LadderConst {
+    D2 m2, m3;  // -2 R^2 and -3 R^2
+};
+WW_HD LadderConst ladder_const(D2 one, const LzMod &m, double rp) {
+    // R 2^32, squared: R^2 2^64 / R = R^2
+    const D2 r2 = lz_canonical(lz_sqr(small_start(1ull << 32, one, m.p, rp), m), m.p);
+    const D2 zero = {0, 0};
+    const D2 t2 = m2_dbl(r2, m.p);
+    LadderConst c;
+    c.m2 = m2_sub(zero, t2, m.p);
+    c.m3 = m2_sub(c.m2, r2, m.p);
+    return c;
+}
+
+// One Lucas step on (e, o) = (W at the even, at the odd of the indices k,
+// k+1): W_2k+1 = W_k W_k+1 - 3 is always the odd one, and the even one is
+// W_2k = W_k^2 - 2 or W_2k+2, the square of e or of o by the bit and the
+// parity of k.  Against two squarings and their difference (V_2k+1 =
+// V_2k+2 - V_2k) the product costs a cross product more and saves the
+// difference with its two corrections, whose operands would have to be
+// canonical.
+WW_HD void lucas_step(D2 &e, D2 &o, bool &kodd, bool bit, const LadderConst &c, const LzMod &m) {
+    const D2 s = sel(bit == kodd, e, o);
+    o = lz_mul_add(e, o, c.m3, m);
+    e = lz_sqr_add(s, c.m2, m);
     kodd = bit;
 }
 
-// 2 V_n+1 - V_n for the ladder's final (e, o) at k = n, n even (n = p +- 1):
-// e = V_n, and o = y - x of the last step, from k = n/2, is +V_n+1 when n/2
-// is even (bit 1 of n clear) and -V_n+1 when it is odd.
-WW_HD D2 eo_finish(D2 e, D2 o, u64 n, u64 p) {
-    const D2 zero = {0, 0};
-    const D2 t = m2_dbl(o, p);
-    return m2_sub(((n >> 1) & 1) ? m2_sub(zero, t, p) : t, e, p);
+// F_n = (2 W_j+1 - 3 W_j) / 5 for n = 2j: 5 is a unit mod p^2 since p has no
+// factor below 127.
+WW_HD D2 lucas_finish(D2 e, D2 o, bool jodd, u64 p, u64 q) {
+    const D2 a = lz_canonical(sel(jodd, o, e), p);  // W_j
+    const D2 b = lz_canonical(sel(jodd, e, o), p);  // W_j+1
+    const D2 d = m2_sub(b, a, p);
+    return m2_div5(m2_redc(m2_sub(m2_dbl(d, p), a, p), p, q), p);
 }
 
-// F_{p-(p|5)} mod p^2 as canonical digits.  The reference walks the
-// (F_k, F_{k-1}) doubling ladder, two squarings and a product per bit
-// (wallsunsun.cl:242-300).  Here the Lucas numbers V_k = L_k run a ladder
-// on (V_k, V_{k+1}) with two squarings per bit:
-//   V_2k = V_k^2 - 2(-1)^k,  V_2k+2 = V_k+1^2 + 2(-1)^k,  V_2k+1 = V_2k+2 - V_2k,
-// and F_n = (2 V_{n+1} - V_n) / 5 gives the same residue exactly (5 is a
-// unit mod p^2 since p has no factor below 127).  The ladder starts from
-// the top six bits of n (ladder_start) and keeps its pair as (V at the even
-// index, V at the odd index up to sign), eo_step; -DWW_NO_EO_LADDER keeps
-// (V_k, V_k+1) instead.
-template <class A>
-WW_HD D2 wss_digits_t(u64 p, u64 q, D2 one) {
-    const A ar(p, q);
-    const u32 pm5 = (u32)(p % 5);
-    const u64 n = (pm5 == 2 || pm5 == 3) ? p + 1 : p - 1;  // p - (p|5)
-    const D2 zero = {0, 0};
-    const D2 two = m2_dbl(one, p);
-    const D2 mtwo = m2_sub(zero, two, p);
-    const int i0 = top_bit(n) - 6;
-    const u32 k0 = (u32)(n >> (i0 + 1));
+// 2^((p-1)/2) mod p^2 as canonical digits (wieferich.cl:219-245).
+WW_HD D2 wieferich_digits(u64 p, u64 q, D2 one) {
+    const LzMod m = lz_mod(p, q);
     const double rp = 1.0 / (double)p;
-    const D2 a = m2_small(lucas_small(k0), one, p, rp);      // V_k0
-    const D2 b = m2_small(lucas_small(k0 + 1), one, p, rp);  // V_k0+1
-    bool odd = k0 & 1u;      // parity of the ladder index k
-    u64 nb = n << (63 - i0);  // bit i of n at bit 63 in step i
-#if !defined(WW_NO_EO_LADDER)
-    D2 e = sel(odd, b, a), o = sel(odd, a, b);
-    for (int i = i0; i >= 0; --i) {
-        const bool bit = (long long)nb < 0;
-        nb <<= 1;
-        eo_step(ar, e, o, odd, bit, two, mtwo, p);
+    const int steps = ladder_steps(lucas_index(p));
+    const u64 f = wieferich_windows(p >> 1, steps);
+    D2 w = small_start(1ull << (f >> steps), one, p, rp);
+    int pos = (steps + kWBits - 1) / kWBits * kWBits;  // the window's low bit, once it is taken
+    int i = steps;
+    while (i > 0) {
+        pos -= kWBits;
+        const u32 d = window_digit(f, pos, i);
+        if (i - pos == kWBits) {  // written out: 1 543 against 1 536 M primes/s
+            w = lz_sqr(w, m);
+            w = lz_sqr(w, m);
+            w = lz_sqr(w, m);
+            w = lz_sqr(w, m);
+            w = lz_sqr(w, m);
+            i = pos;
+        }
+        for (; i > pos; --i) w = lz_sqr(w, m);
+        w = lz_shift(w, d, m);
     }
-    const D2 t = ar.redc(eo_finish(e, o, n, p));
-#else
-    D2 va = a, vb = b;
-    for (int i = i0; i >= 0; --i) {
-        const bool bit = (long long)nb < 0;
-        nb <<= 1;
-        const D2 c = sel(odd, two, mtwo);  // -2(-1)^k
-        const D2 v2k = m2_add(ar.sqr(va), c, p);
-        const D2 v2k2 = m2_sub(ar.sqr(vb), c, p);
-        const D2 v2k1 = m2_sub(v2k2, v2k, p);
-        va = sel(bit, v2k1, v2k);
-        vb = sel(bit, v2k2, v2k1);
-        odd = bit;
-    }
-    const D2 t = ar.redc(m2_sub(m2_dbl(vb, p), va, p));
-#endif
-    return m2_div5(t, p);
+    return m2_redc(lz_canonical(w, p), p, q);
 }
 
-// Both tests in one loop: each iteration advances the Lucas ladder by one
-// bit of p - (p|5) and the Wieferich powering by one bit of (p-1)/2.  The
-// ladder step uses two squarings instead of a squaring and a product:
-//   V_2k = V_k^2 - 2(-1)^k,  V_2k+2 = V_k+1^2 + 2(-1)^k,
-//   V_2k+1 = V_2k+2 - V_2k   (the recurrence V_m+1 = V_m + V_m-1),
-// so the three products of an iteration are squarings, independent of each
-// other, and no operand has to be selected before multiplying.  Both start
-// from their top bits (ladder_start), the Wieferich powering at most one
-// bit after the ladder; the Lucas pair is kept as eo_step's (e, o).
-template <class A>
-WW_HD void both_digits_t(u64 p, u64 q, D2 one, D2 &s_out, D2 &c_out) {
-    const A ar(p, q);
-    const u32 pm5 = (u32)(p % 5);
-    const u64 n = (pm5 == 2 || pm5 == 3) ? p + 1 : p - 1;
-    const u64 e = p >> 1;
-    const D2 zero = {0, 0};
-    const D2 two = m2_dbl(one, p);
-    const D2 mtwo = m2_sub(zero, two, p);
-    const LadderStart st = ladder_start(p, n, one);
-    D2 w = st.w;
-    bool odd = st.odd;
-    // bit i of n and of e at bit 63 in step i (shifts by one instead of by i)
-    u64 nb = n << (63 - st.i0);
-    u64 eb = e << (63 - st.i0);
-#if !defined(WW_NO_EO_LADDER)
-    D2 le = sel(odd, st.b, st.a), lo = sel(odd, st.a, st.b);
-    for (int i = st.i0; i >= 0; --i) {
-        const bool bit = (long long)nb < 0;
-        const bool ebit = (long long)eb < 0;
-        nb <<= 1;
-        eb <<= 1;
-        eo_step(ar, le, lo, odd, bit, two, mtwo, p);
-        if (i <= st.iw) {
-            w = ar.sqr(w);
-#if defined(WW_W_WINDOW)
-            if (((st.iw - i) & 3) == 3) w = m2_mul_pow2(w, (u32)(e >> i) & 15u, p, st.rp);
-#else
-            w = sel(ebit, m2_dbl(w, p), w);
-#endif
-        }
+// F_{p-(p|5)} mod p^2 as canonical digits (wallsunsun.cl:242-300).
+WW_HD D2 wss_digits(u64 p, u64 q, D2 one) {
+    const LzMod m = lz_mod(p, q);
+    const double rp = 1.0 / (double)p;
+    const u64 j = lucas_index(p);
+    const int steps = ladder_steps(j);
+    const LadderConst c = ladder_const(one, m, rp);
+    const u32 k0 = (u32)(j >> steps);
+    bool kodd = k0 & 1u;
+    D2 e = small_start(lucas_even(k0 + (k0 & 1u)), one, p, rp);
+    D2 o = small_start(lucas_even(k0 | 1u), one, p, rp);
+    u64 jb = j << (63 - steps) << 1;  // the next bit at bit 63
+    for (int i = steps; i > 0; --i) {
+        lucas_step(e, o, kodd, (long long)jb < 0, c, m);
+        jb <<= 1;
     }
-#if defined(WW_W_WINDOW)
-    const int rest = (st.iw + 1) & 3;
-    if (rest) w = m2_mul_pow2(w, (u32)e & ((1u << rest) - 1u), p, st.rp);
-#endif
-    s_out = ar.redc(w);
-    c_out = m2_div5(ar.redc(eo_finish(le, lo, n, p)), p);
-#else
-    D2 a = st.a, b = st.b;
-    for (int i = st.i0; i >= 0; --i) {
-        const bool bit = (long long)nb < 0;
-        const bool ebit = (long long)eb < 0;
-        nb <<= 1;
-        eb <<= 1;
-        const D2 a2 = ar.sqr(a);
-        const D2 b2 = ar.sqr(b);
-        if (i <= st.iw) {
-            w = ar.sqr(w);
-#if defined(WW_W_WINDOW)
-            // every fourth bit from iw down: w *= 2^v for the group's four bits
-            if (((st.iw - i) & 3) == 3) w = m2_mul_pow2(w, (u32)(e >> i) & 15u, p, st.rp);
-#else
-            w = sel(ebit, m2_dbl(w, p), w);
-#endif
-        }
-        const D2 c = sel(odd, two, mtwo);     // -2(-1)^k
-        const D2 v2k = m2_add(a2, c, p);      // V_2k
-        const D2 v2k2 = m2_sub(b2, c, p);     // V_2k+2
-        const D2 v2k1 = m2_sub(v2k2, v2k, p); // V_2k+1
-        a = sel(bit, v2k1, v2k);
-        b = sel(bit, v2k2, v2k1);
-        odd = bit;
-    }
-#if defined(WW_W_WINDOW)
-    const int rest = (st.iw + 1) & 3;  // the last, partial group of bits
-    if (rest) w = m2_mul_pow2(w, (u32)e & ((1u << rest) - 1u), p, st.rp);
-#endif
-    s_out = ar.redc(w);
-    c_out = m2_div5(ar.redc(m2_sub(m2_dbl(b, p), a, p)), p);
-#endif
+    return lucas_finish(e, o, kodd, p, q);
 }
 
-WW_HD D2 wieferich_digits(u64 p, u64 q, D2 one) { return wieferich_digits_t<WW_ARITH>(p, q, one); }
-WW_HD void both_digits(u64 p, u64 q, D2 one, D2 &s, D2 &c) { both_digits_t<WW_ARITH>(p, q, one, s, c); }
-WW_HD D2 wss_digits(u64 p, u64 q, D2 one) { return wss_digits_t<WW_ARITH>(p, q, one); }
+// Both in one loop: the three products of a step are independent.
+WW_HD void both_digits(u64 p, u64 q, D2 one, D2 &s_out, D2 &c_out) {
+    const LzMod m = lz_mod(p, q);
+    const double rp = 1.0 / (double)p;
+    const u64 j = lucas_index(p);
+    const int steps = ladder_steps(j);
+    const u64 f = wieferich_windows(p >> 1, steps);
+    const LadderConst c = ladder_const(one, m, rp);
+    const u32 k0 = (u32)(j >> steps);
+    bool kodd = k0 & 1u;
+    D2 e = small_start(lucas_even(k0 + (k0 & 1u)), one, p, rp);
+    D2 o = small_start(lucas_even(k0 | 1u), one, p, rp);
+    D2 w = small_start(1ull << (f >> steps), one, p, rp);
+    u64 jb = j << (63 - steps) << 1;
+    int pos = (steps + kWBits - 1) / kWBits * kWBits;
+    int i = steps;
+    while (i > 0) {
+        pos -= kWBits;
+        const u32 d = window_digit(f, pos, i);
+        for (; i > pos; --i) {
+            lucas_step(e, o, kodd, (long long)jb < 0, c, m);
+            w = lz_sqr(w, m);
+            jb <<= 1;
+        }
+        w = lz_shift(w, d, m);
+    }
+    s_out = m2_redc(lz_canonical(w, p), p, q);
+    c_out = lucas_finish(e, o, kodd, p, q);
+}
 
 // ------------------------------------------------------------ classification
 
