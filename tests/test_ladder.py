@@ -66,3 +66,35 @@ def test_gpu_ladders_mixed_sizes(ww, keep):
                 ctx.wieferich()
                 ctx.wallsunsun()
             assert ctx.counters()["checksum"] == total
+
+
+SMALL = [3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61, 67, 71, 73, 79, 83, 89, 97, 101, 103, 107,
+         109, 113]
+
+
+def strong_prp2(n: int) -> bool:
+    if any(n % r == 0 for r in SMALL):
+        return False
+    t = ((n - 1) & -(n - 1)).bit_length() - 1
+    x = pow(2, (n - 1) >> t, n)
+    if x in (1, n - 1):
+        return True
+    for _ in range(t - 1):
+        x = x * x % n
+        if x == n - 1:
+            return True
+    return False
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", list(range(8, 65)))
+def test_gpu_prp_test_around_powers_of_two(ww, k):
+    """Both sides of 2^k: numbers of two lengths in one warp, and n - 1 with
+    every 2-adic valuation up to k (2^32 + 1 is a strong pseudoprime)."""
+    lo = max(127, 2**k - 2000)
+    hi = min(2**64 - 1, 2**k + 2000)
+    expect = [n for n in range(lo | 1, hi, 2) if strong_prp2(n)]
+    with ww.Context(0, max_prps=1 << 12) as ctx:
+        ctx.clear_segment()
+        ctx.sieve_prp(lo, hi)
+        assert sorted(int(v) for v in ctx.prps()) == expect

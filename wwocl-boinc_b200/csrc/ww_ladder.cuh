@@ -252,6 +252,88 @@ WW_HD D2 lz_shift(D2 x, u32 d, const LzMod &m) {
     return r;
 }
 
+// 2^e by left-to-right squaring, for the Wieferich test and the PRP test: the
+// bits of e below its start are multiplied in five at a time as 2^(d-32),
+// 0 <= d < 32 (one-word Montgomery steps: 6 instructions a bit for two digits
+// where a conditional doubling takes 18, 3 against 11 for one).  With
+// f = e + sum of 32^(w+1) over the windows w, e is the start f >> steps
+// (below 48 where e >> steps is below 32) times 2^steps plus the sum of
+// (d_w - 32) 32^w.
+constexpr int kWinBits = 5;
+WW_HD u64 power_windows(u64 e, int steps) {
+    // 32 + 32^2 + ... for ceil(steps / 5) windows
+    const int n = (steps + kWinBits - 1) / kWinBits;
+    const u64 ones = 0x0842108421084210ull << 1;  // bits 5, 10, ..., 60
+    return e + (ones & ((2ull << (kWinBits * n)) - 1));
+}
+// The digit of the window at bit pos, below bit i (the top window is short).
+WW_HD u32 window_digit(u64 f, int pos, int i) { return (u32)(f >> pos) & ((1u << (i - pos)) - 1u); }
+
+#if defined(__CUDACC__)
+// A^2 / R mod n
+__device__ __forceinline__ u64 lz_sqr1(u64 a, const LzMod &m) {
+    u64 u;
+    u32 neg;
+    return lz_low(lz_square(a), m, u, neg);
+}
+
+// The base-2 strong probable-prime test (sprp2) for a whole warp: all 32
+// lanes call it, and lanes with act false test the first active lane's number
+// and return false.  The bits of n-1 above every lane's lowest set bit t touch
+// neither the value at bit t nor the -1 check, so the powering takes them in
+// windows of five, with the same number of squarings in every lane; from the
+// warp's largest t down (some six squarings) it goes bit by bit, as sprp2
+// does, and keeps the value at bit t and whether -1 appears below it.
+__device__ __forceinline__ bool sprp2_warp(u64 n, bool act, u64 &q_out) {
+    const u32 live = __ballot_sync(0xffffffffu, act);
+    if (live == 0) {
+        q_out = 0;
+        return false;
+    }
+    const u64 src = __shfl_sync(0xffffffffu, n, __ffs((int)live) - 1);
+    n = act ? n : src;
+    const u64 q = inv64(n);
+    q_out = q;
+    const LzMod m = lz_mod(n, q);
+    const u64 one = r_mod(n);
+    const u64 mone = n - one;
+    const u64 nm1 = n - 1;
+    const int t = __ffsll((long long)nm1) - 1;  // >= 1: n is odd
+    const int tw = (int)__reduce_max_sync(0xffffffffu, (unsigned)t);
+    const int top = (int)__reduce_max_sync(0xffffffffu, (unsigned)(63 - __clzll((long long)nm1)));
+    const int steps = top - tw > 5 ? top - tw - 5 : 0;
+    const u64 f = power_windows(nm1 >> tw >> 1, steps);
+    const u32 e0 = (u32)(f >> steps);
+    u64 a = one, unused;
+    if (e0) a = mod_est(one >> (64 - e0), one << e0, n, 1.0 / (double)n, unused);
+    int i = steps, pos = (steps + kWinBits - 1) / kWinBits * kWinBits;
+    const u32 n0 = (u32)n, n1 = (u32)(n >> 32);
+    while (i > 0) {
+        pos -= kWinBits;
+        const u32 d = window_digit(f, pos, i);
+        for (; i > pos; --i) a = lz_sqr1(a, m);
+        // a 2^(d-32): one 32-bit Montgomery step (lz_shift)
+        const u32 w = ((u32)a << d) * (u32)q;
+        u32 neg;
+        const u64 r = lz_sub(a >> (32 - d), (u64)w * n1 + (((u64)w * n0) >> 32), neg);
+        a = lz_addp(r, neg, m);
+    }
+    u64 ebits = nm1 << (63 - tw);  // bit tw at bit 63
+    u64 at_t = 0;
+    bool m1 = false;
+    for (i = tw; i >= 1; --i) {
+        a = lz_sqr1(a, m);
+        const u64 d = add_mod(a, a, n);
+        a = ((long long)ebits < 0) ? d : a;
+        ebits <<= 1;
+        at_t = (i == t) ? a : at_t;
+        m1 |= (i < t) & (a == mone);
+    }
+    const bool ok = (at_t == one) | (at_t == mone) | m1;
+    return act && ok;
+}
+#endif
+
 // x1 < 2p made canonical
 WW_HD D2 lz_canonical(D2 x, u64 p) {
     if (x.d1 >= p) x.d1 -= p;

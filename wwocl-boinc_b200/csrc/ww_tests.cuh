@@ -117,22 +117,6 @@ WW_HD int ladder_steps(u64 j) {
     return top > 4 ? top - 4 : 0;
 }
 
-// Wieferich: 2^e by left-to-right squaring; the bits of e are multiplied in
-// five at a time as 2^(d-32), 0 <= d < 32 (lz_shift: two one-word Montgomery
-// steps, 6 instructions a bit where a conditional doubling of two digits
-// takes 18).  With f = e + sum of 32^(w+1) over the windows w, e is the start
-// f >> steps (below 48) times 2^steps plus the sum of (d_w - 32) 32^w.
-constexpr int kWBits = 5;
-WW_HD u64 wieferich_windows(u64 e, int steps) {
-    // 32 + 32^2 + ... for ceil(steps / 5) windows: 32 (32^n - 1) / 31
-    const int n = (steps + kWBits - 1) / kWBits;
-    const u64 ones = 0x0842108421084210ull << 1;  // bits 5, 10, ..., 60
-    return e + (ones & ((2ull << (kWBits * n)) - 1));
-}
-
-// The digit of the window at bit pos, below bit i (the top window is short).
-WW_HD u32 window_digit(u64 f, int pos, int i) { return (u32)(f >> pos) & ((1u << (i - pos)) - 1u); }
-
 // L R mod p^2 as canonical digits for L < 2^48.  For p >= 2^62 the quotient
 // of L 2^64 by p is below 2^50 and mod_est's estimate within 2^-1 of it (three
 // roundings of 2^-53 and those of (double)p), so its correction by one is
@@ -189,14 +173,14 @@ WW_HD D2 wieferich_digits(u64 p, u64 q, D2 one) {
     const LzMod m = lz_mod(p, q);
     const double rp = 1.0 / (double)p;
     const int steps = ladder_steps(lucas_index(p));
-    const u64 f = wieferich_windows(p >> 1, steps);
+    const u64 f = power_windows(p >> 1, steps);
     D2 w = small_start(1ull << (f >> steps), one, p, rp);
-    int pos = (steps + kWBits - 1) / kWBits * kWBits;  // the window's low bit, once it is taken
+    int pos = (steps + kWinBits - 1) / kWinBits * kWinBits;  // the window's low bit, once it is taken
     int i = steps;
     while (i > 0) {
-        pos -= kWBits;
+        pos -= kWinBits;
         const u32 d = window_digit(f, pos, i);
-        if (i - pos == kWBits) {  // written out: 1 543 against 1 536 M primes/s
+        if (i - pos == kWinBits) {  // written out: 1 543 against 1 536 M primes/s
             w = lz_sqr(w, m);
             w = lz_sqr(w, m);
             w = lz_sqr(w, m);
@@ -235,7 +219,7 @@ WW_HD void both_digits(u64 p, u64 q, D2 one, D2 &s_out, D2 &c_out) {
     const double rp = 1.0 / (double)p;
     const u64 j = lucas_index(p);
     const int steps = ladder_steps(j);
-    const u64 f = wieferich_windows(p >> 1, steps);
+    const u64 f = power_windows(p >> 1, steps);
     const LadderConst c = ladder_const(one, m, rp);
     const u32 k0 = (u32)(j >> steps);
     bool kodd = k0 & 1u;
@@ -243,10 +227,10 @@ WW_HD void both_digits(u64 p, u64 q, D2 one, D2 &s_out, D2 &c_out) {
     D2 o = small_start(lucas_even(k0 | 1u), one, p, rp);
     D2 w = small_start(1ull << (f >> steps), one, p, rp);
     u64 jb = j << (63 - steps) << 1;
-    int pos = (steps + kWBits - 1) / kWBits * kWBits;
+    int pos = (steps + kWinBits - 1) / kWinBits * kWinBits;
     int i = steps;
     while (i > 0) {
-        pos -= kWBits;
+        pos -= kWinBits;
         const u32 d = window_digit(f, pos, i);
         for (; i > pos; --i) {
             lucas_step(e, o, kodd, (long long)jb < 0, c, m);
