@@ -98,3 +98,21 @@ def test_gpu_prp_test_around_powers_of_two(ww, k):
         ctx.clear_segment()
         ctx.sieve_prp(lo, hi)
         assert sorted(int(v) for v in ctx.prps()) == expect
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [2**11 - 2, 2**11 + 2, 40_000, 1_212_416, 1_300_000, 9_700_000, 77_594_624,
+                                   77_600_000, 2**26 - 1, 2**26 + 1, 310_400_000, 311_000_000, 620_000_000, 2**29])
+@pytest.mark.parametrize("low", [127, 10**9 + 1, 2**64 - 2**31 + 3])
+def test_gpu_small_segments_equal_fixed_ones(ww, low, width):
+    """The segment size chosen by width against the fixed narrow segments, at
+    the widths where the size, the rounds or the marks change: same list."""
+    with ww.Context(0, max_prps=ww.prp_count_bound(low, low + width) + 1000) as ctx:
+        lists = []
+        for shape, depth in ((0, 28), (2, 20)):
+            ctx.set_sieve_shape(shape)
+            ctx.set_sieve_depth(depth)
+            ctx.clear_segment()
+            ctx.sieve_prp(low, low + width)
+            lists.append(np.sort(ctx.prps()))
+        assert np.array_equal(lists[0], lists[1])

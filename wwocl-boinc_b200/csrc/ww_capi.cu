@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <chrono>
+#include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -284,32 +285,70 @@ cudaError_t sieve_slots(int *slots) {
     return cudaSuccess;
 }
 
+// About how many primes are below b.
+double primes_below(double b) { return b < 256.0 ? (b < 127.0 ? 0.0 : 54.0) : b / (log(b) - 1.1); }
+
+// Rows of the deep table worth their start-up in a segment of `numbers`
+// numbers below `high`: the primes below about B with B ln B = 7 times the
+// segment, since the primes near B spare 0.56 / (B ln B) of its numbers
+// their PRP test each (7 measured best on widths 1e6 to 2^28 among 3, 5, 7,
+// 10, 20, 33 and 60: 1e8 numbers in 687 us, at 33 in 843 us); and none above
+// the square root of `high`, whose multiples a smaller prime marks.  Any
+// count gives the same PRPs.
+int deep_rows_for(double numbers, uint64_t high) {
+    const double x = 7.0 * numbers;
+    double b = x / log(x / 10.0);
+    const double root = sqrt((double)high) + 1.0;
+    if (b > root) b = root;
+    const double n = primes_below(b) - 30.0;
+    return n < 0.0 ? 0 : n < (double)kDeepUse ? (int)n : kDeepUse;
+}
+
 template <class G>
-int launch_sieve_shape(uint64_t low, uint64_t high, uint64_t span, const PrpOut &out, u64 *cursor,
+int launch_sieve_shape(uint64_t low, uint64_t high, uint64_t span, int words, const PrpOut &out, u64 *cursor,
                        const DeepRow *deep, cudaStream_t stream, const u32 *marks) {
-    const uint64_t per = 2ull * G::kOdd;
+    const uint64_t per = 64ull * (uint64_t)words;
     const uint64_t nseg = span / per + (span % per ? 1 : 0);
     int slots = 0;
     WW_CU(sieve_slots<G>(&slots));
     const uint64_t grid = nseg < (uint64_t)slots ? nseg : (uint64_t)slots;
+    SievePlan plan;
+    plan.words = words;
+    plan.deep_n = deep_rows_for((double)per, high);
+    // one prime in 512 numbers of the segment by a whole warp (1e8 numbers:
+    // 687 us, with half as many 698, with a quarter 711)
+    plan.warp_n = per / 512 < (uint64_t)kDeepWarpPrimes ? (int)(per / 512) : kDeepWarpPrimes;
+    const size_t smem = (size_t)words * 4 + (size_t)G::kWarps * kQueueCap * 4;
     if (cursor) WW_CU(cudaMemsetAsync(cursor, 0, sizeof(u64), stream));
-    k_sieve_prp<G><<<(unsigned)grid, G::kThreads, G::kSmem, stream>>>(low, high, nseg, out, cursor, deep, marks);
+    k_sieve_prp<G><<<(unsigned)grid, G::kThreads, smem, stream>>>(low, high, nseg, out, cursor, deep, marks, plan);
     WW_CHECK_LAUNCH();
     return WW_OK;
 }
 
 // One sieve launch over [low, high).  shape 1: the wide segments, 2: the
-// narrow ones, 0: the wide shape once the range gives each of its resident
-// CTAs a segment, below that the narrow one, which has twice the segments.
+// narrow ones, 0: by the range's width -- the wide shape once the range
+// gives each of its resident CTAs two segments (2^29 numbers: 2.70 ms against
+// 2.98 ms from one segment on; 2^30: the same), below that the small shape
+// with its segments cut so that every resident CTA gets the same number of
+// them, one up to 3.1e8 numbers.  Near 2^64, against the narrow shape down to
+// the last number: 1e5 numbers 23 us (424), 1e6 33 (910), 1.6e7 171 (982),
+// 1e8 640 (1 243), 2^28 1 465 us (2 050).
 int launch_sieve_range(uint64_t low, uint64_t high, const PrpOut &out, u64 *cursor, const DeepRow *deep,
                        cudaStream_t stream, const u32 *marks, int shape) {
     const uint64_t span = high - (low & ~1ull);
-    int wide_slots = 0;
-    WW_CU(sieve_slots<SieveWide>(&wide_slots));
-    const uint64_t wide_segs = span / (2ull * SieveWide::kOdd) + 1;
-    if (shape == 1 || (shape == 0 && wide_segs >= (uint64_t)wide_slots))
-        return launch_sieve_shape<SieveWide>(low, high, span, out, cursor, deep, stream, marks);
-    return launch_sieve_shape<SieveNarrow>(low, high, span, out, cursor, deep, stream, marks);
+    int slots = 0;
+    WW_CU(sieve_slots<SieveWide>(&slots));
+    if (shape == 1 || (shape == 0 && span / (2ull * SieveWide::kOdd) + 1 >= 2ull * (uint64_t)slots))
+        return launch_sieve_shape<SieveWide>(low, high, span, SieveWide::kWords, out, cursor, deep, stream, marks);
+    if (shape == 2)
+        return launch_sieve_shape<SieveNarrow>(low, high, span, SieveNarrow::kWords, out, cursor, deep, stream, marks);
+    WW_CU(sieve_slots<SieveSmall>(&slots));
+    const uint64_t per_slot = span / (64ull * (uint64_t)slots) + 1;  // words
+    const uint64_t rounds = (per_slot + SieveSmall::kMaxWords - 1) / SieveSmall::kMaxWords;
+    uint64_t words = (per_slot + rounds - 1) / rounds;
+    words = words <= 256 ? (words + 7) / 8 * 8 : (words + 31) / 32 * 32;
+    if (words < (uint64_t)SieveSmall::kMinWords) words = SieveSmall::kMinWords;
+    return launch_sieve_shape<SieveSmall>(low, high, span, (int)words, out, cursor, deep, stream, marks);
 }
 
 }  // namespace
@@ -359,7 +398,13 @@ int launch_sieve(uint64_t low, uint64_t high, int32_t wheelidx, uint64_t *g_prim
         // whole segments of the wide shape (2^19 odd numbers) cover either shape's reads
         const u64 words = ((nodd + SieveWide::kOdd - 1) / SieveWide::kOdd) * (u64)SieveWide::kWords;
         if (words > large->words) return set_err("mark bitmap too small"), WW_ERR_STATE;
-        int rc = launch_deep_fill(a + 1, nodd, large->table, large->bits, words, st);
+        // a narrow piece takes the table's smaller primes only, below 0.4 of
+        // its width: a row's start costs the same whatever the width (7e7
+        // numbers 477 us, with the whole table 545; 2^28 and up the same)
+        DeepLarge rows = large->table;
+        const double worth = primes_below(0.4 * (double)(b - a)) - (double)kDeepUse;
+        if (worth < (double)rows.n) rows.n = worth > 0.0 ? (u32)worth : 0;
+        int rc = launch_deep_fill(a + 1, nodd, rows, large->bits, words, st);
         if (rc) return rc;
         rc = launch_sieve_range(lo, b, out, cursor, deep, st, large->bits, shape);
         if (rc) return rc;

@@ -28,6 +28,7 @@ struct SieveGeom {
     static constexpr int kWordsPerThread = W / T;
     static constexpr size_t kSmem = (size_t)W * 4 + (size_t)(T / 32) * kQueueCap * 4;
     static_assert(W % T == 0 && W % 32 == 0 && T % 32 == 0, "sieve geometry");
+    static constexpr bool kRuntime = false;
 };
 // 2^20 numbers per segment for 512 threads, two CTAs and 32 warps per SM.
 // Each doubling of the segment halves the deep primes' per-segment start-up
@@ -44,6 +45,21 @@ typedef SieveGeom<WW_SIEVE_WIDE_WORDS, WW_SIEVE_WIDE_THREADS> SieveWide;
 // 2^19 numbers for 256 threads: twice the segments, for ranges that would
 // not give every resident CTA of the wide shape a segment.
 typedef SieveGeom<8192, 256> SieveNarrow;
+// Segments of 32 to 8192 words (2^11 to 2^19 numbers, chosen at the launch)
+// for 256 threads: ranges too narrow for the wide shape.  A multiple of 8
+// words, of 32 from 256 on, so that a warp's share is whole words.
+struct SieveSmall {
+    static constexpr int kThreads = 256, kWarps = 8;
+    static constexpr int kMinWords = 32, kMaxWords = 8192;
+    static constexpr size_t kSmem = (size_t)kMaxWords * 4 + (size_t)kWarps * kQueueCap * 4;
+    static constexpr bool kRuntime = true;
+};
+// What a launch's segments are sieved with: words per segment (SieveSmall
+// alone reads it), how many rows of the deep table, and how many of those
+// are marked one warp per prime.
+struct SievePlan {
+    int words, deep_n, warp_n;
+};
 
 #ifndef WW_TEST_THREADS
 #define WW_TEST_THREADS 256
@@ -120,18 +136,19 @@ __device__ __forceinline__ void step_hit(u32 &j0) {
 // get its address as an argument.  Host code asks for it per device.
 const DeepRow *deep_rows_device();
 
-// Mark the odd multiples n = r*k of the deep primes in the segment, except
-// those with k = 1 (mod ord_r(2)) (ww_deep.cuh says why).  The smallest
-// primes have the most multiples: each of the first kDeepWarpPrimes primes
-// is marked by a whole warp (lane l takes the multiples l, l + 32, ...; k
-// then grows by 64 per step), the rest one prime per thread, so no thread
-// holds the others at the next barrier.
+// Mark the odd multiples n = r*k of the first deep_n deep primes in the
+// segment, except those with k = 1 (mod ord_r(2)) (ww_deep.cuh says why).
+// The smallest primes have the most multiples: each of the first warp_n
+// primes is marked by a whole warp (lane l takes the multiples l, l + 32,
+// ...; k then grows by 64 per step), the rest one prime per thread, so no
+// thread holds the others at the next barrier.
 constexpr int kDeepWarpPrimes = 512;
 
 __device__ __forceinline__ void deep_mark(u64 first, u32 nvalid, u32 *bitmap, int tid, int nthreads,
-                                          const DeepRow *__restrict__ deep) {
+                                          const DeepRow *__restrict__ deep, int deep_n = kDeepUse,
+                                          int warp_n = kDeepWarpPrimes) {
     const int lane = tid & 31, warp = tid >> 5, nwarps = nthreads >> 5;
-    for (int i = warp; i < kDeepWarpPrimes && i < kDeepUse; i += nwarps) {
+    for (int i = warp; i < warp_n && i < deep_n; i += nwarps) {
         const DeepRow e = deep[i];
         u32 j0, km0;
         deep_start(first, e, j0, km0);
@@ -143,7 +160,7 @@ __device__ __forceinline__ void deep_mark(u64 first, u32 nvalid, u32 *bitmap, in
             if (km >= e.o) km -= e.o;
         }
     }
-    for (int i = kDeepWarpPrimes + tid; i < kDeepUse; i += nthreads) {
+    for (int i = warp_n + tid; i < deep_n; i += nthreads) {
         const DeepRow e = deep[i];
         u32 j, km;
         deep_start(first, e, j, km);

@@ -37,14 +37,24 @@ namespace ww {
 // one that found every cursor of the library's pool busy) they stride over
 // the segments.  marks (optional): the large deep primes' marks of the whole
 // launch, bit j of word w = odd number b0 + 2(32 w + j) + 1 (ww_bucket.cu),
-// ORed into each segment's bitmap.
+// ORed into each segment's bitmap.  plan: SievePlan.
 template <class G>
 __global__ void __launch_bounds__(G::kThreads, WW_SIEVE_MINB_THREADS / G::kThreads) k_sieve_prp(u64 lo, u64 hi, u64 nseg, PrpOut out,
                                                                               u64 *cursor, const DeepRow *deep,
-                                                                              const u32 *__restrict__ marks) {
-    extern __shared__ u32 sieve_smem[];  // G::kSmem bytes
+                                                                              const u32 *__restrict__ marks,
+                                                                              SievePlan plan) {
+    extern __shared__ u32 sieve_smem[];
+    int words, chunk_words;  // of a segment, and of the share a warp takes of it at a time
+    if constexpr (G::kRuntime) {
+        words = plan.words;
+        chunk_words = min(32, words / G::kWarps);
+    } else {
+        words = G::kWords;
+        chunk_words = 32;
+    }
+    const u64 odd = 32ull * (u64)words;  // odd numbers of a segment
     u32 *bitmap = sieve_smem;
-    u32(*queue)[kQueueCap] = reinterpret_cast<u32(*)[kQueueCap]>(sieve_smem + G::kWords);
+    u32(*queue)[kQueueCap] = reinterpret_cast<u32(*)[kQueueCap]>(sieve_smem + words);
     __shared__ u32 s_chunk;
     __shared__ u64 s_seg;
     const u64 b0 = lo & ~1ull;
@@ -59,20 +69,22 @@ __global__ void __launch_bounds__(G::kThreads, WW_SIEVE_MINB_THREADS / G::kThrea
         seg = s_seg;
     }
     while (seg < nseg) {
-        const u64 seg_off = seg * (u64)(2 * G::kOdd);
+        const u64 seg_off = seg * 2 * odd;
         const u64 rem_span = span - seg_off;  // > 0
-        const u64 nvalid = (rem_span / 2 < (u64)G::kOdd) ? rem_span / 2 : (u64)G::kOdd;
+        const u64 nvalid = rem_span / 2 < odd ? rem_span / 2 : odd;
 
         // ---- pre-sieve 3..113 on this thread's contiguous words
-        {
-            const int w0 = threadIdx.x * G::kWordsPerThread;
+        const int wpt = (words + G::kThreads - 1) / G::kThreads;
+        const int w0 = threadIdx.x * wpt;
+        const int w1 = G::kRuntime ? min(w0 + wpt, words) : w0 + wpt;
+        if (!G::kRuntime || w0 < words) {
             const u64 n0 = b0 + seg_off + 64ull * (u64)w0 + 1;  // may wrap past 2^64 beyond hi
-            const u32 *seg_marks = marks ? marks + seg * (u64)G::kWords : nullptr;
+            const u32 *seg_marks = marks ? marks + seg * (u64)words : nullptr;
 #define WW_J0(R) u32 j##R = first_hit<R>(n0);
             WW_FOR_SMALL_PRIMES(WW_J0)
 #undef WW_J0
 #pragma unroll 4
-            for (int w = w0; w < w0 + G::kWordsPerThread; ++w) {
+            for (int w = w0; w < w1; ++w) {
                 u32 m = seg_marks ? seg_marks[w] : 0u;
 #define WW_MASK(R) m |= prime_mask<R>(j##R); step_hit<R>(j##R);
                 WW_FOR_SMALL_PRIMES(WW_MASK)
@@ -91,10 +103,11 @@ __global__ void __launch_bounds__(G::kThreads, WW_SIEVE_MINB_THREADS / G::kThrea
 
         // ---- deep sieve 113 < r < 2^WW_DEEP_BITS, sparing possible pseudoprimes
         const u64 nbase = b0 + seg_off + 1;
-        deep_mark(nbase, (u32)nvalid, bitmap, threadIdx.x, G::kThreads, deep);
+        deep_mark(nbase, (u32)nvalid, bitmap, threadIdx.x, G::kThreads, deep,
+                  G::kRuntime ? plan.deep_n : kDeepUse, G::kRuntime ? plan.warp_n : kDeepWarpPrimes);
         __syncthreads();
 
-        // ---- warps take 32-word chunks dynamically (so they reach the next
+        // ---- warps take chunks of 32 words (or fewer) dynamically (so they reach the next
         // barrier together), compact the survivors with ballot/popc into a
         // warp queue and PRP-test them 32 at a time
         u32 *q = queue[warp];
@@ -103,10 +116,10 @@ __global__ void __launch_bounds__(G::kThreads, WW_SIEVE_MINB_THREADS / G::kThrea
             u32 chunk = 0;
             if (lane == 0) chunk = atomicAdd(&s_chunk, 1u);
             chunk = __shfl_sync(0xffffffffu, chunk, 0);
-            const bool more = chunk < (u32)(G::kWords / 32);
+            const bool more = (int)chunk * chunk_words < words;
             if (more) {
-                const int w = chunk * 32 + lane;
-                u32 cand = ~bitmap[w];
+                const int w = chunk * chunk_words + lane;
+                u32 cand = !G::kRuntime || lane < chunk_words ? ~bitmap[w] : 0u;
                 const int cnt = __popc(cand);
                 int incl = cnt;
 #pragma unroll
