@@ -3,6 +3,7 @@
 // simpleCL layer (main.cpp:51-90, simpleCL.c:352-719).
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
@@ -273,15 +274,22 @@ int ww_launch_getsegprimes(uint64_t low, uint64_t high, int32_t wheelidx, uint64
 namespace {
 
 // Resident CTAs of k_sieve_prp<G> on the current device (the dynamic
-// shared memory limit is raised first).
+// shared memory limit is raised first; asked of the driver once per device).
 template <class G>
 cudaError_t sieve_slots(int *slots) {
-    cudaError_t e = cudaFuncSetAttribute(k_sieve_prp<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::kSmem);
+    static std::atomic<int> known[kCursorPoolDevices];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const bool keep = dev >= 0 && dev < kCursorPoolDevices;
+    if (keep && (*slots = known[dev].load(std::memory_order_acquire)) > 0) return cudaSuccess;
+    e = cudaFuncSetAttribute(k_sieve_prp<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::kSmem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sieve_prp<G>, G::kThreads, G::kSmem);
     if (e != cudaSuccess) return e;
     *slots = sm_count() * (per_sm < 1 ? 1 : per_sm);
+    if (keep) known[dev].store(*slots, std::memory_order_release);
     return cudaSuccess;
 }
 
@@ -498,6 +506,15 @@ struct DevCounters {
 
 __global__ void k_set_count(unsigned int *pc, unsigned int v) { pc[0] = v; }
 
+// ww_clear_results in one launch: everything but the segment's count
+__global__ void k_clear_results(DevCounters *c) {
+    c->checksum = 0;
+    c->total = 0;
+    c->resultcount = 0;
+    c->primecount[1] = 0;
+    c->overflow = 0;
+}
+
 }  // namespace
 
 namespace ww {
@@ -701,10 +718,8 @@ int ww_get_buffers(ww_ctx *c, ww_buffers *b) {
 
 int ww_clear_results(ww_ctx *c) {
     if (!c) return set_err("null ctx"), WW_ERR_ARG;
-    int rc = ww_launch_clearresult((uint64_t *)&c->dc->checksum, &c->dc->resultcount, (uint64_t *)&c->dc->total,
-                                   c->dc->primecount, c->stream);
-    if (rc) return rc;
-    WW_CU(cudaMemsetAsync(&c->dc->overflow, 0, sizeof(unsigned int), c->stream));
+    k_clear_results<<<1, 1, 0, c->stream>>>(c->dc);
+    WW_CHECK_LAUNCH();
     return WW_OK;
 }
 
@@ -921,10 +936,14 @@ static int wait_event(cudaEvent_t ev, uint32_t timeout_ms) {
             set_err("cudaEventQuery: %s", cudaGetErrorString(e));
             return WW_ERR_CUDA;
         }
-        const auto dt = std::chrono::steady_clock::now() - t0;
-        if (timeout_ms && std::chrono::duration_cast<std::chrono::milliseconds>(dt).count() >= timeout_ms)
+        const long long us =
+            std::chrono::duration_cast<std::chrono::microseconds>(std::chrono::steady_clock::now() - t0).count();
+        if (timeout_ms && us / 1000 >= (long long)timeout_ms)
             return set_err("timed out after %u ms", timeout_ms), WW_ERR_TIMEOUT;
-        std::this_thread::sleep_for(std::chrono::microseconds(200));
+        // poll through the first 200 us, then sleep a sixteenth of the time
+        // waited so far, up to 200 us: a fixed 200 us was most of the wait
+        // for a short range (262 us for one that takes 60)
+        if (us >= 200) std::this_thread::sleep_for(std::chrono::microseconds(us < 3200 ? us / 16 : 200));
     }
 }
 

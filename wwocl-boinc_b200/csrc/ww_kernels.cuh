@@ -174,14 +174,18 @@ constexpr u64 kIdlePrime = 0xFFFFFFFFFFFFFFC5ull;  // 2^64 - 59
 // before the launch) each warp pulls one unit at a time, so warps that run
 // ahead take more of the work and all finish together; without one (a
 // launch captured into a graph, or one that found every cursor of the
-// library's pool busy) the grid strides.
+// library's pool busy) the grid strides.  Units that do not outnumber the
+// grid's warps go one to a warp, neighbours to different SMs, without the
+// cursor, whose atomics from every warp of the grid would take longer than a
+// step of the ladders.
 template <class F>
 __device__ __forceinline__ void for_each_unit(u64 n, u64 *cursor, F &&f) {
     const int lane = threadIdx.x & 31;
-    u64 unit = ((u64)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    u64 unit = (u64)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
     const u64 stride = ((u64)gridDim.x * blockDim.x) >> 5;
+    const bool pull = cursor && n > stride;
     for (;;) {
-        if (cursor) {
+        if (pull) {
             if (lane == 0) unit = atomicAdd((unsigned long long *)cursor, 1ull);
             unit = __shfl_sync(0xffffffffu, unit, 0);
         }

@@ -38,6 +38,10 @@ class Hit(C.Structure):
                 ("quot", C.c_int32), ("pad", C.c_int32)]
 
 
+_HIT_DTYPE = np.dtype([("p", np.uint64), ("result", np.int32), ("rem", np.int32), ("quot", np.int32),
+                       ("pad", np.int32)])
+
+
 class Counters(C.Structure):
     _fields_ = [("checksum", C.c_uint64), ("total_prp_count", C.c_uint64),
                 ("result_count", C.c_uint32), ("seg_prp_count", C.c_uint32),
@@ -425,10 +429,11 @@ class Context:
 
     def hits(self) -> list[tuple[int, int, int, int]]:
         cap = self.max_hits
-        arr = (Hit * cap)()
+        rows = np.empty(cap, _HIT_DTYPE)
         n = C.c_uint32(0)
-        check(_L.ww_read_hits(self.h, arr, cap, C.byref(n)), "ww_read_hits")
-        return [(arr[i].p, arr[i].result, arr[i].rem, arr[i].quot) for i in range(min(n.value, cap))]
+        check(_L.ww_read_hits(self.h, rows.ctypes.data_as(C.POINTER(Hit)), cap, C.byref(n)), "ww_read_hits")
+        rows = rows[: min(n.value, cap)]
+        return list(zip(*(rows[f].tolist() for f in ("p", "result", "rem", "quot"))))
 
     def prps(self) -> np.ndarray:
         cnt = self.counters()["seg_prp_count"]
@@ -462,7 +467,7 @@ class Context:
             start = stop
         self.sync()
         c = self.counters()
-        c["hits"] = [] if c["overflow"] & 2 else self.hits()
+        c["hits"] = [] if c["overflow"] & 2 or not c["result_count"] else self.hits()
         return c
 
 
