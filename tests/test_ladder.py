@@ -116,3 +116,32 @@ def test_gpu_small_segments_equal_fixed_ones(ww, low, width):
             ctx.sieve_prp(low, low + width)
             lists.append(np.sort(ctx.prps()))
         assert np.array_equal(lists[0], lists[1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("widths", [[1], [2**13 - 1, 2**13 + 1], [100_000], [300_001] * 5, [40_000_000, 999, 1_000_000],
+                                    [50_000] * 300, [2**28 + 5, 7, 2**20]])
+@pytest.mark.parametrize("cfg", [(16384, 512, 1, 0), (4096, 128, 1, 0), (16384, 1024, 1, 0), (8192, 256, 8, 0)])
+def test_gpu_cut_tiles_equal_units_alone(ww, widths, cfg):
+    """Batches whose tiles are cut small: each unit as alone on the plain path,
+    and its tiles still counted in the configuration's full ones; the same
+    ranges as requests (one step may take the first's last tile and the next
+    one's) and through the allocation-free entry (tests/test_zz_no_alloc.py
+    covers its own sizes)."""
+    rng = random.Random(len(widths) + cfg[1])
+    starts = [rng.randrange(127, 2**64 - 2**29) for _ in widths]
+    units = [(a, a + w) for a, w in zip(starts, widths)]
+    with ww.Context(0, max_prps=ww.prp_count_bound(0, max(widths)) + 1000) as ctx:
+        batch = ww.Batch(ctx)
+        batch.set_config(*cfg)
+        got = batch.run(units)
+        alone = [ctx.run_range(a, b) for a, b in units]
+        want = [(r["checksum"], r["total_prp_count"], r["result_count"]) for r in alone]
+        assert [(r["checksum"], r["prp_count"], r["hits"]) for r in got] == want
+        assert [r["tiles_done"] for r in got] == [-(-w // (64 * cfg[0])) for w in widths]
+        server = ww.Server(ctx, prp_pool_bytes=1 << 28, max_active=8)
+        server.submit([(i, a, b) for i, (a, b) in enumerate(units)])
+        done = sorted(server.drain(), key=lambda r: r["id"])
+        assert [(r["checksum"], r["prp_count"], r["hits"]) for r in done] == want
+        assert [r["prps_stored"] for r in done] == [w[1] for w in want]
+        server.close()

@@ -94,6 +94,8 @@ ww_batch_cfg default_cfg() { return ww_batch_cfg{16384, 512, 1, 0}; }
 // the request server's unless the caller chose one for the context: the same
 // tile, with one CTA per SM per step (server_init)
 ww_batch_cfg default_serve_cfg() { return default_cfg(); }
+// and no tile above 2^18 numbers, which keeps the steps' ends even
+constexpr u32 kServeMaxWords = 4096;
 
 }  // namespace
 
@@ -111,6 +113,7 @@ struct BatchState {
     UnitState *h_units = nullptr;  // pinned mirror of d_units
     u64 *h_first = nullptr;        // pinned tile table
     u32 n_units = 0;
+    u64 tile = 0;                  // numbers of a full tile of the submitted batch
     cudaGraphExec_t exec = nullptr;
     bool tuned = false;
     ww_batch_cfg cfg = default_cfg();
@@ -178,6 +181,17 @@ int ensure_capacity(BatchState &b, u32 n_units, u32 hit_cap) {
     return WW_OK;
 }
 
+// A finished unit's tiles counted in full ones, whatever they were cut into.
+u32 full_tiles(const UnitState &u, u64 tile) {
+    if (u.tiles_done < u.n_tiles) return (u32)((u64)u.tiles_done * 64 * u.words / tile);
+    const u64 w = u.end - u.start;
+    return (u32)(w / tile + (w % tile ? 1 : 0));
+}
+
+void fill_deep_n(BatchArgs &a) {
+    for (int k = 0; k < kTileSizes; ++k) a.deep_n[k] = deep_rows_for(64.0 * (kTileMinWords << k), ~0ull);
+}
+
 BatchArgs make_args(BatchState &b, u32 n, u64 n_tiles) {
     BatchArgs a;
     a.units = b.d_units;
@@ -185,7 +199,7 @@ BatchArgs make_args(BatchState &b, u32 n, u64 n_tiles) {
     a.tile_first = b.d_first;
     a.n_tiles = n_tiles;
     a.next_tile = b.d_next;
-    a.epoch_tiles = b.d_epoch;
+    a.epoch_words = b.d_epoch;
     a.budget = 0;
     a.hit_p = b.d_hit_p;
     a.hit_result = b.d_hit_res;
@@ -196,6 +210,7 @@ BatchArgs make_args(BatchState &b, u32 n, u64 n_tiles) {
     a.hit_capacity = b.hit_cap;
     a.overflow = b.d_overflow;
     a.deep = deep_rows_device();  // callers check it before launching
+    fill_deep_n(a);
     return a;
 }
 
@@ -219,20 +234,28 @@ int run_batch(ww_ctx *ctx, BatchState &b, const ww_unit *units, uint32_t n, cons
               u64 *n_tiles_out) {
     const int dev = ctx_device(ctx);
     cudaStream_t st = (cudaStream_t)ctx_stream(ctx);
-    const u64 tile = 64ull * (u64)e.seg_words;
     int rc = ensure_capacity(b, n ? n : 1, b.hit_cap ? b.hit_cap : 1u << 16);
     if (rc) return rc;
+    int grid = 0;
+    rc = launch_grid(e, dev, &grid);
+    if (rc) return rc;
     WW_CU(cudaStreamSynchronize(st));  // the pinned mirror may still feed a previous launch
-    u64 acc = 0;
+    double left = 0;  // numbers from unit i on: the last units get smaller tiles, so the CTAs end together
     for (uint32_t i = 0; i < n; ++i) {
         if (units[i].end < units[i].start || (units[i].end > units[i].start && units[i].start < 127))
             return set_err("unit %u: bad range [%llu, %llu)", i, (unsigned long long)units[i].start,
                            (unsigned long long)units[i].end), WW_ERR_ARG;
+        left += (double)(units[i].end - units[i].start);
+    }
+    u64 acc = 0;
+    for (uint32_t i = 0; i < n; ++i) {
         UnitState &u = b.h_units[i];
         memset(&u, 0, sizeof u);
         u.start = units[i].start;
         u.end = units[i].end;
-        const u64 w = units[i].end - units[i].start;
+        u.words = tile_words(left, grid, (u32)e.seg_words);
+        const u64 w = units[i].end - units[i].start, tile = 64ull * u.words;
+        left -= (double)w;
         u.n_tiles = w / tile + (w % tile ? 1 : 0);
         u.active = 1;
         b.h_first[i] = acc;
@@ -240,10 +263,8 @@ int run_batch(ww_ctx *ctx, BatchState &b, const ww_unit *units, uint32_t n, cons
     }
     b.h_first[n] = acc;
     b.n_units = n;
+    b.tile = 64ull * (u64)e.seg_words;
     *n_tiles_out = acc;
-    int grid = 0;
-    rc = launch_grid(e, dev, &grid);
-    if (rc) return rc;
     const BatchArgs a = make_args(b, n, acc);
     if (!a.deep) return WW_ERR_CUDA;
 
@@ -350,7 +371,7 @@ int ww_batch_collect(ww_ctx *ctx, ww_unit_result *out, uint32_t n, uint32_t *hit
         out[i].checksum = bs->h_units[i].checksum;
         out[i].prp_count = bs->h_units[i].prp_count;
         out[i].hits = bs->h_units[i].hits;
-        out[i].tiles_done = bs->h_units[i].tiles_done;
+        out[i].tiles_done = full_tiles(bs->h_units[i], bs->tile);
     }
     if (hit_count) *hit_count = hc[0];
     if (hc[1] & 2) return set_err("%u hits, buffer holds %u", hc[0], bs->hit_cap), WW_ERR_HIT_OVERFLOW;
@@ -458,7 +479,8 @@ struct ServerSlot {
 struct ServerState {
     ww_server_cfg cfg{};
     const CfgEntry *e = nullptr;
-    int grid = 0;
+    int grid = 0;              // resident CTAs
+    int step_tiles = 0;        // full tiles' worth of words a step hands out
     UnitState *d_slots = nullptr, *h_slots = nullptr;
     u64 *pool = nullptr;
     u32 *d_epoch = nullptr, *d_hit_count = nullptr, *d_overflow = nullptr;
@@ -586,12 +608,11 @@ int server_init(ServerState &s, ww_ctx *ctx, const ww_server_cfg *cfg) {
     int per_sm = 0, sms = 0;
     WW_CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, s.e->serve_kernel, s.e->threads, s.e->smem));
     WW_CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx_device(ctx)));
-    // a step hands out one tile per CTA, and small requests wait about one
-    // step: with 512 threads' worth of CTAs per SM (one 512-thread tile) the
-    // step is half as long as with the two an SM can hold, for 7 % less
-    // throughput, which the server's load leaves room for
-    const int step_per_sm = std::max(1, std::min(per_sm, 512 / s.e->threads));
-    s.grid = step_per_sm * sms;
+    // a step hands out as many words as 512 threads' worth of full tiles per
+    // SM have (one 512-thread tile), cut into smaller tiles for every CTA an
+    // SM can hold: small requests wait about one step, so it stays short
+    s.step_tiles = std::max(1, std::min(per_sm, 512 / s.e->threads)) * sms;
+    s.grid = per_sm * sms;
     const u32 n = cfg->max_active, h = cfg->max_hits;
     WW_CU(cudaMalloc(&s.d_slots, (size_t)n * sizeof(UnitState)));
     WW_CU(cudaMallocHost(&s.h_slots, (size_t)n * sizeof(UnitState)));
@@ -674,12 +695,22 @@ int ww_server_step(ww_ctx *ctx, ww_request_result *done, uint32_t cap, uint32_t 
     *ndone = 0;
     ServerState &s = *sv;
     cudaStream_t st = (cudaStream_t)ctx_stream(ctx);
-    const u64 tile = 64ull * (u64)s.e->seg_words;
     s.done_prps.clear();
 
     // ---- admission: FIFO while a slot and PRP-buffer memory are free
     const u32 n = s.cfg.max_active;
     bool changed = false;
+    // a request's tiles are cut by all the work at hand: small ones only while
+    // there is too little for every CTA
+    double left = 0;
+    if (!s.queue.empty()) {
+        for (u32 k = 0; k < n; ++k)
+            if (s.slots[k].busy) {
+                const UnitState &u = s.h_slots[k];
+                left += 64.0 * u.words * (double)(u.n_tiles - std::min(u.next_tile, u.n_tiles));
+            }
+        for (const ServerReq &q : s.queue) left += (double)(q.r.end - q.r.start);
+    }
     for (u32 k = 0; k < n && !s.queue.empty(); ++k) {
         if (s.slots[k].busy) continue;
         const ServerReq &q = s.queue.front();
@@ -702,6 +733,8 @@ int ww_server_step(ww_ctx *ctx, ww_request_result *done, uint32_t cap, uint32_t 
         u.start = q.r.start;
         u.end = q.r.end;
         const u64 w = q.r.end - q.r.start;
+        u.words = std::min(tile_words(left, s.grid, (u32)s.e->seg_words), kServeMaxWords);
+        const u64 tile = 64ull * u.words;
         u.n_tiles = w / tile + (w % tile ? 1 : 0);
         u.active = 1;
         if (s.cfg.store_prps) {
@@ -722,13 +755,14 @@ int ww_server_step(ww_ctx *ctx, ww_request_result *done, uint32_t cap, uint32_t 
     // latency from 134 ms (equal round-robin shares) to 93 ms at the same
     // p50.  Until a step has been timed, the order is that of submission.
     const double wave_s = s.tile_s > 0 ? s.tile_s : 1e-6;
-    const double grid_slots = (double)std::max(1, s.grid);
+    const double wave_words = (double)std::max(1, s.step_tiles) * s.e->seg_words;
     u32 n_order = 0;
     std::vector<std::pair<double, u32>> by_deadline;
     by_deadline.reserve(active);
     for (u32 k = 0; k < n; ++k)
         if (s.slots[k].busy)
-            by_deadline.emplace_back(s.slots[k].t_submit + 2.0 * (double)s.h_slots[k].n_tiles / grid_slots * wave_s, k);
+            by_deadline.emplace_back(s.slots[k].t_submit +
+                                         2.0 * (double)s.h_slots[k].n_tiles * s.h_slots[k].words / wave_words * wave_s, k);
     std::sort(by_deadline.begin(), by_deadline.end());
     for (const auto &d : by_deadline) s.h_order[n_order++] = d.second;
     if (changed)
@@ -743,12 +777,13 @@ int ww_server_step(ww_ctx *ctx, ww_request_result *done, uint32_t cap, uint32_t 
     a.n_units = n;
     a.order = s.d_order;
     a.n_order = n_order;
-    a.epoch_tiles = s.d_epoch;
-    // whole waves of the resident CTAs: a partial last wave would leave most
+    a.epoch_words = s.d_epoch;
+    fill_deep_n(a);
+    // whole waves of the step's tiles: a partial last wave would leave most
     // SMs idle while its few tiles finish
-    const u32 g = (u32)s.grid;
-    if (s.cfg.epoch_tiles == 0) a.budget = g;  // one wave
-    else a.budget = s.cfg.epoch_tiles < g ? s.cfg.epoch_tiles : std::max(1u, (s.cfg.epoch_tiles + g / 2) / g) * g;
+    const u64 g = (u64)s.step_tiles, asked = s.cfg.epoch_tiles;
+    const u64 tiles = asked == 0 ? g : asked < g ? asked : std::max<u64>(1, (asked + g / 2) / g) * g;
+    a.budget = (u32)std::min<u64>(tiles * (u64)s.e->seg_words, 0xf0000000ull);
     a.hit_p = s.d_hit_p;
     a.hit_result = s.d_hit_res;
     a.hit_rem = s.d_hit_rem;
@@ -759,10 +794,14 @@ int ww_server_step(ww_ctx *ctx, ww_request_result *done, uint32_t cap, uint32_t 
     a.overflow = s.d_overflow;
     a.deep = deep_rows_device();
     if (!a.deep) return WW_ERR_CUDA;
-    const int grid = std::min<int>(s.grid, (int)a.budget);
-    u64 tiles_before = 0;
+    u32 least = (u32)s.e->seg_words;  // no more CTAs than the budget has tiles
     for (u32 k = 0; k < n; ++k)
-        if (s.slots[k].busy) tiles_before += std::min(s.h_slots[k].next_tile, s.h_slots[k].n_tiles);
+        if (s.slots[k].busy) least = std::min(least, s.h_slots[k].words);
+    const int grid = (int)std::min<u64>((u64)s.grid, std::max<u32>(1, a.budget / least));
+    u64 words_before = 0;
+    for (u32 k = 0; k < n; ++k)
+        if (s.slots[k].busy)
+            words_before += std::min(s.h_slots[k].next_tile, s.h_slots[k].n_tiles) * s.h_slots[k].words;
     const double t_launch = mono_s();
     s.e->serve_kernel<<<grid, s.e->threads, s.e->smem, st>>>(a);
     WW_CU(cudaGetLastError());
@@ -770,13 +809,14 @@ int ww_server_step(ww_ctx *ctx, ww_request_result *done, uint32_t cap, uint32_t 
     WW_CU(cudaMemcpyAsync(s.h_counts, s.d_hit_count, 4, cudaMemcpyDeviceToHost, st));
     WW_CU(cudaMemcpyAsync(s.h_counts + 1, s.d_overflow, 4, cudaMemcpyDeviceToHost, st));
     WW_CU(cudaStreamSynchronize(st));
-    {  // seconds per wave of tiles, from this step's tiles and time
-        u64 tiles_after = 0;
+    {  // seconds per wave of tiles, from this step's words and time
+        u64 words_after = 0;
         for (u32 k = 0; k < n; ++k)
-            if (s.slots[k].busy) tiles_after += std::min(s.h_slots[k].next_tile, s.h_slots[k].n_tiles);
-        const u64 ran = tiles_after - tiles_before;
+            if (s.slots[k].busy)
+                words_after += std::min(s.h_slots[k].next_tile, s.h_slots[k].n_tiles) * s.h_slots[k].words;
+        const u64 ran = words_after - words_before;
         if (ran) {
-            const double per = (mono_s() - t_launch) / std::ceil((double)ran / grid_slots);
+            const double per = (mono_s() - t_launch) / std::ceil((double)ran / wave_words);
             s.tile_s = s.tile_s > 0 ? 0.8 * s.tile_s + 0.2 * per : per;
         }
     }

@@ -9,9 +9,16 @@
 // the survivors into a warp queue, run the base-2 strong PRP test 32 at a
 // time, and push the PRPs into a second warp queue that feeds the
 // Wieferich and Wall-Sun-Sun tests 32 (or 64 with two primes per thread) at
-// a time.  Checksums and PRP counts go to the tile's unit with one atomic
-// per warp per batch; the sums are order-free, so every unit's checksum is
-// bit-identical to a run of that unit alone.
+// a time.  That queue is kept from tile to tile, each PRP with its unit, and
+// emptied at the end of the launch, so small tiles do not leave test batches
+// half empty.  Checksums and PRP counts go to the unit with one atomic per
+// batch (one per lane where a batch mixes units); the sums are order-free, so
+// every unit's checksum is bit-identical to a run of that unit alone.
+//
+// A unit's tile is at most the configuration's segment and a power of two of
+// words below it (UnitState::words): tiles small enough that the launch has
+// several for every resident CTA, since 2^20-number tiles gave a batch of
+// eight ranges of 1e5 to 1e6 numbers to eight CTAs.
 #pragma once
 
 #include "ww_device.cuh"
@@ -29,8 +36,13 @@ struct UnitState {
     u64 prp_cap;
     u64 prp_written;         // PRPs found (may exceed prp_cap: overflow)
     u32 hits, tiles_done;
-    u32 active, pad;
+    u32 active;
+    u32 words;               // bitmap words of a tile of this unit
 };
+
+// Tiles have kTileMinWords << k words, k < kTileSizes.
+constexpr int kTileMinWords = 128;
+constexpr int kTileSizes = 9;
 
 struct BatchArgs {
     UnitState *units;
@@ -39,9 +51,10 @@ struct BatchArgs {
     const u64 *tile_first;
     u64 n_tiles;
     u64 *next_tile;          // queue head
-    // serving: at most `budget` tiles this launch, handed out in the order of
-    // `order` (slot indices, earliest deadline first; n_order entries)
-    u32 *epoch_tiles;
+    // serving: tiles of about `budget` words in all this launch, handed out in
+    // the order of `order` (slot indices, earliest deadline first; n_order
+    // entries)
+    u32 *epoch_words;
     u32 budget;
     const u32 *order;
     u32 n_order;
@@ -53,6 +66,7 @@ struct BatchArgs {
     u32 hit_capacity;
     u32 *overflow;           // bit 1: hit list overflow, bit 0: a PRP buffer overflowed
     const DeepRow *deep;     // the deep-sieve table (deep_rows_device())
+    int deep_n[kTileSizes];  // its rows used for tiles of kTileMinWords << k words
 };
 
 // A tile configuration: SEG_WORDS bitmap words, THREADS per CTA, PPT batches
@@ -75,16 +89,10 @@ struct BatchCfg {
     // at 64)
     static constexpr int kSmThreads = PPT >= 4 ? THREADS : 1024;
     static constexpr int kMinBlocks = kSmThreads / THREADS > 0 ? kSmThreads / THREADS : 1;
-    static constexpr int kChunks = SEG_WORDS / 32;
-    static constexpr u64 kTileNumbers = 64ull * SEG_WORDS;  // integers per tile
+    static constexpr u64 kTileNumbers = 64ull * SEG_WORDS;  // integers per full tile
     static constexpr int kCandCap = 416;  // as kQueueCap: 31 carried + at most 378 per 32-word chunk
     static constexpr int kPrpCap = 32 * PPT + 32;
     static_assert(SEG_WORDS % THREADS == 0, "words per thread");
-};
-
-struct WarpAcc {
-    u64 checksum;
-    u32 count;
 };
 
 __device__ __forceinline__ void emit_batch_hit(const BatchArgs &a, u32 unit, u64 p, int result, int rem, int quot) {
@@ -101,24 +109,22 @@ __device__ __forceinline__ void emit_batch_hit(const BatchArgs &a, u32 unit, u64
     atomicAdd(&a.units[unit].hits, 1u);
 }
 
-// Wieferich + WSS on the warp's PRP queue entries [base, base + 32*PPT);
-// `valid` lanes only.  Adds to the warp's accumulator (lane 0 holds it).
+// Wieferich + WSS on the first n_valid of 32*PPT entries of the warp's PRP
+// queue, each added to its own unit.
 template <int PPT, bool JOINT>
-__device__ __forceinline__ void test_batch(const u64 *qp, int n_valid, u32 unit, const BatchArgs &a,
-                                           WarpAcc &acc) {
+__device__ __forceinline__ void test_batch(const u64 *qp, const u32 *qu, int n_valid, const BatchArgs &a) {
     const int lane = threadIdx.x & 31;
-    u64 sum = 0;
-    u32 cnt = 0;
 #pragma unroll
     for (int k = 0; k < PPT; ++k) {
         const int idx = k * 32 + lane;
         const bool act = idx < n_valid;
         const u64 p = act ? qp[idx] : 0xFFFFFFFFFFFFFFC5ull;  // 2^64-59, a harmless prime
+        const u32 unit = act ? qu[idx] : 0u;
         const u64 q = inv64(p);
         const D2 one = m2_one(p);
         // one after the other: fewer registers live at once, so the
         // 512-thread tiles fit 64 registers (two CTAs, 32 warps per SM);
-        // the joint loop has three independent squarings per step
+        // the joint loop has three independent products per step
         D2 s, c;
         if (JOINT) {
             both_digits(p, q, one, s, c);
@@ -126,39 +132,59 @@ __device__ __forceinline__ void test_batch(const u64 *qp, int n_valid, u32 unit,
             s = wieferich_digits(p, q, one);
             c = wss_digits(p, q, one);
         }
+        u64 sum = 0;
         if (act) {
-            sum += (s.d1 & 0xffffffffull) + (c.d1 & 0xffffffffull);
-            ++cnt;
+            sum = (s.d1 & 0xffffffffull) + (c.d1 & 0xffffffffull);
             int rem, quot_w, res, quot_s;
             const bool hw = wieferich_classify(p, s, rem, quot_w);
             const bool hs = wss_classify(p, c, res, quot_s);
             if (hw) emit_batch_hit(a, unit, p, 1093, rem, quot_w);  // as the wieferich kernel would
             if (hs) emit_batch_hit(a, unit, p, res, 0, quot_s);     // as the wallsunsun kernel would
         }
+        // one atomic a batch when its PRPs are of one unit
+        const u32 live = __ballot_sync(0xffffffffu, act);
+        if (live == 0) continue;
+        const u32 unit0 = __shfl_sync(0xffffffffu, unit, __ffs((int)live) - 1);
+        if (__all_sync(0xffffffffu, !act || unit == unit0)) {
+            sum = warp_sum(sum);
+            if (lane == 0) {
+                atomicAdd((unsigned long long *)&a.units[unit0].checksum, (unsigned long long)sum);
+                atomicAdd((unsigned long long *)&a.units[unit0].prp_count, (unsigned long long)__popc(live));
+            }
+        } else if (act) {
+            atomicAdd((unsigned long long *)&a.units[unit].checksum, (unsigned long long)sum);
+            atomicAdd((unsigned long long *)&a.units[unit].prp_count, 1ull);
+        }
     }
-    sum = warp_sum(sum);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-    if (lane == 0) {
-        acc.checksum += sum;
-        acc.count += cnt;
-    }
+}
+
+// Bitmap words of a unit's tiles: the largest power of two, up to the
+// configuration's segment, that cuts `numbers` (what is left of the launch
+// from this unit on) into kTileRounds tiles for each of `slots` resident CTAs.
+#ifndef WW_TILE_ROUNDS
+#define WW_TILE_ROUNDS 2
+#endif
+constexpr double kTileRounds = WW_TILE_ROUNDS;
+inline u32 tile_words(double numbers, int slots, u32 seg_words) {
+    u32 w = seg_words;
+    while (w > (u32)kTileMinWords && 64.0 * w * kTileRounds * slots > numbers) w /= 2;
+    return w;
 }
 
 template <class Cfg>
 constexpr size_t batch_smem_bytes() {
-    return (size_t)Cfg::kWarps * Cfg::kPrpCap * 8 + (size_t)Cfg::kWords * 4 +
+    return (size_t)Cfg::kWarps * Cfg::kPrpCap * 12 + (size_t)Cfg::kWords * 4 +
            (size_t)Cfg::kWarps * Cfg::kCandCap * 4;
 }
 
 // Hand out the next tile.  Batch: the global queue head over the static
 // tile table.  Serving: the first unit in the host's priority order that
-// has tiles left, through that unit's own cursor, at most `budget` tiles per
-// launch; the loop is bounded by the number of units, so an exhausted queue
-// ends the kernel instead of spinning.
+// has tiles left, through that unit's own cursor, until the tiles handed out
+// this launch have `budget` words; the loop is bounded by the number of
+// units, so an exhausted queue ends the kernel instead of spinning.
 template <bool SERVE>
 __device__ __forceinline__ bool next_tile(const BatchArgs &a, u32 &unit, u64 &tile) {
-    if (!SERVE) {
+    if constexpr (!SERVE) {
         const u64 t = atomicAdd((unsigned long long *)a.next_tile, 1ull);
         if (t >= a.n_tiles) return false;
         u32 lo = 0, hi = a.n_units;  // last k with tile_first[k] <= t
@@ -169,35 +195,45 @@ __device__ __forceinline__ bool next_tile(const BatchArgs &a, u32 &unit, u64 &ti
         unit = lo;
         tile = t - a.tile_first[lo];
         return true;
-    }
-    if (atomicAdd(a.epoch_tiles, 1u) >= a.budget) return false;
-    for (u32 i = 0; i < a.n_order; ++i) {
-        const u32 k = a.order[i];
-        UnitState &u = a.units[k];
-        // the cursor is read past L1 (other CTAs move it); a stale value
-        // only costs an atomic that finds the unit exhausted
-        if (!u.active || *(volatile u64 *)&u.next_tile >= u.n_tiles) continue;
-        const u64 t = atomicAdd((unsigned long long *)&u.next_tile, 1ull);
-        if (t < u.n_tiles) {
-            unit = k;
-            tile = t;
-            return true;
+    } else {
+        // a tile counts when it is taken, not when it is looked for: CTAs that
+        // race for a unit's last tile would use up the budget
+        if (*(volatile u32 *)a.epoch_words >= a.budget) return false;
+        for (u32 i = 0; i < a.n_order; ++i) {
+            const u32 k = a.order[i];
+            UnitState &u = a.units[k];
+            // the cursor is read past L1 (other CTAs move it); a stale value
+            // only costs an atomic that finds the unit exhausted
+            if (!u.active || *(volatile u64 *)&u.next_tile >= u.n_tiles) continue;
+            const u64 t = atomicAdd((unsigned long long *)&u.next_tile, 1ull);
+            if (t < u.n_tiles) {
+                atomicAdd(a.epoch_words, u.words);
+                unit = k;
+                tile = t;
+                return true;
+            }
         }
+        return false;
     }
-    return false;
 }
 
 template <class Cfg, bool SERVE>
 __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) k_tiles(BatchArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
+    constexpr size_t kPrps = (size_t)Cfg::kWarps * Cfg::kPrpCap;
     u64(*prpq)[Cfg::kPrpCap] = reinterpret_cast<u64(*)[Cfg::kPrpCap]>(smem);
-    u32 *bitmap = reinterpret_cast<u32 *>(smem + (size_t)Cfg::kWarps * Cfg::kPrpCap * 8);
-    u32(*candq)[Cfg::kCandCap] =
-        reinterpret_cast<u32(*)[Cfg::kCandCap]>(smem + (size_t)Cfg::kWarps * Cfg::kPrpCap * 8 + Cfg::kWords * 4);
+    u32 *bitmap = reinterpret_cast<u32 *>(smem + kPrps * 8);
+    u32(*candq)[Cfg::kCandCap] = reinterpret_cast<u32(*)[Cfg::kCandCap]>(smem + kPrps * 8 + Cfg::kWords * 4);
+    u32(*unitq)[Cfg::kPrpCap] = reinterpret_cast<u32(*)[Cfg::kPrpCap]>(
+        smem + kPrps * 8 + Cfg::kWords * 4 + (size_t)Cfg::kWarps * Cfg::kCandCap * 4);
     __shared__ u64 s_lo, s_hi;
-    __shared__ u32 s_unit, s_chunk, s_ok;
+    __shared__ u32 s_unit, s_chunk, s_ok, s_words;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
+    u32 *cq = candq[warp];
+    u64 *pq = prpq[warp];
+    u32 *uq = unitq[warp];
+    int pn = 0;  // PRPs in the warp's queue, kept from tile to tile
 
     for (;;) {
         if (threadIdx.x == 0) {
@@ -207,31 +243,37 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) k_tiles(BatchA
             s_ok = next_tile<SERVE>(a, k, t) ? 1u : 0u;
             if (s_ok) {
                 const UnitState &u = a.units[k];
-                const u64 tlo = u.start + t * Cfg::kTileNumbers;
+                const u64 numbers = 64ull * (u64)u.words;
+                const u64 tlo = u.start + t * numbers;
                 const u64 room = u.end - tlo;
                 s_unit = k;
+                s_words = u.words;
                 s_lo = tlo;
-                s_hi = room > Cfg::kTileNumbers ? tlo + Cfg::kTileNumbers : u.end;
+                s_hi = room > numbers ? tlo + numbers : u.end;
             }
         }
         __syncthreads();
-        if (!s_ok) return;
+        if (!s_ok) break;
         const u64 lo = s_lo, hi = s_hi;
         const u32 unit = s_unit;
+        const int words = (int)s_words;
+        const int chunk_words = min(32, words / Cfg::kWarps);  // a warp's share at a time
 
         // ---- pre-sieve 3..113 over [lo, hi): bit j of the tile is b0 + 2j + 1
         const u64 b0 = lo & ~1ull;
         const u64 span = hi - b0;
-        const u64 nvalid = span / 2 < (u64)(Cfg::kWords * 32) ? span / 2 : (u64)(Cfg::kWords * 32);
-        {
-            constexpr int kWpt = Cfg::kWords / Cfg::kThreads;
-            const int w0 = threadIdx.x * kWpt;
+        const u64 odd = 32ull * (u64)words;
+        const u64 nvalid = span / 2 < odd ? span / 2 : odd;
+        const int wpt = (words + Cfg::kThreads - 1) / Cfg::kThreads;
+        const int w0 = threadIdx.x * wpt;
+        if (w0 < words) {
+            const int w1 = min(w0 + wpt, words);
             const u64 n0 = b0 + 64ull * (u64)w0 + 1;
 #define WW_J0(R) u32 j##R = first_hit<R>(n0);
             WW_FOR_SMALL_PRIMES(WW_J0)
 #undef WW_J0
 #pragma unroll 2
-            for (int w = w0; w < w0 + kWpt; ++w) {
+            for (int w = w0; w < w1; ++w) {
                 u32 m = 0;
 #define WW_MASK(R) m |= prime_mask<R>(j##R); step_hit<R>(j##R);
                 WW_FOR_SMALL_PRIMES(WW_MASK)
@@ -248,14 +290,12 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) k_tiles(BatchA
 
         // ---- deep sieve 113 < r < 2^WW_DEEP_BITS, sparing possible pseudoprimes
         const u64 nbase = b0 + 1;
-        deep_mark(nbase, (u32)nvalid, bitmap, threadIdx.x, Cfg::kThreads, a.deep);
+        deep_mark(nbase, (u32)nvalid, bitmap, threadIdx.x, Cfg::kThreads, a.deep,
+                  a.deep_n[__ffs(words) - __ffs(kTileMinWords)], min(words / 8, kDeepWarpPrimes));
         __syncthreads();
 
-        // ---- chunks of 32 words, taken dynamically by the warps
-        u32 *cq = candq[warp];
-        u64 *pq = prpq[warp];
-        int cn = 0, pn = 0;
-        WarpAcc acc = {0, 0};
+        // ---- chunks of 32 words (or fewer), taken dynamically by the warps
+        int cn = 0;
         // one PRP test per lane; passing numbers go to the warp's PRP queue,
         // which feeds the Wieferich + WSS batches
         auto sprp_step = [&](u32 j, bool act) {
@@ -264,7 +304,10 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) k_tiles(BatchA
             const bool pass = prp_test_warp(n, act, q);
             const u32 ballot = __ballot_sync(0xffffffffu, pass);
             const u32 rank = __popc(ballot & ((1u << lane) - 1u));
-            if (pass) pq[pn + rank] = n;
+            if (pass) {
+                pq[pn + rank] = n;
+                uq[pn + rank] = unit;
+            }
             if (a.units[unit].prp_out && ballot) {  // the range's PRP buffer (serving)
                 u64 base = 0;
                 if (lane == 0)
@@ -280,7 +323,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) k_tiles(BatchA
             __syncwarp();
             while (pn >= 32 * Cfg::kPpt) {
                 pn -= 32 * Cfg::kPpt;
-                test_batch<Cfg::kPpt, Cfg::kJoint>(pq + pn, 32 * Cfg::kPpt, unit, a, acc);
+                test_batch<Cfg::kPpt, Cfg::kJoint>(pq + pn, uq + pn, 32 * Cfg::kPpt, a);
                 __syncwarp();
             }
         };
@@ -288,10 +331,10 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) k_tiles(BatchA
             u32 chunk = 0;
             if (lane == 0) chunk = atomicAdd(&s_chunk, 1u);
             chunk = __shfl_sync(0xffffffffu, chunk, 0);
-            const bool more = chunk < (u32)Cfg::kChunks;
+            const bool more = (int)chunk * chunk_words < words;
             if (more) {
-                const int w = chunk * 32 + lane;
-                u32 cand = ~bitmap[w];
+                const int w = chunk * chunk_words + lane;
+                u32 cand = lane < chunk_words ? ~bitmap[w] : 0u;
                 const int c = __popc(cand);
                 int incl = c;
 #pragma unroll
@@ -320,20 +363,13 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) k_tiles(BatchA
             }
             if (!more) break;
         }
-        if (pn > 0) {
-            test_batch<Cfg::kPpt, Cfg::kJoint>(pq, pn, unit, a, acc);
-            pn = 0;
-        }
-        if (lane == 0 && acc.count) {
-            atomicAdd((unsigned long long *)&a.units[unit].checksum, (unsigned long long)acc.checksum);
-            atomicAdd((unsigned long long *)&a.units[unit].prp_count, (unsigned long long)acc.count);
-        }
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
             atomicAdd(&a.units[unit].tiles_done, 1u);
         }
     }
+    if (pn > 0) test_batch<Cfg::kPpt, Cfg::kJoint>(pq, uq, pn, a);
 }
 
 }  // namespace ww

@@ -271,6 +271,29 @@ int ww_launch_getsegprimes(uint64_t low, uint64_t high, int32_t wheelidx, uint64
 
 }  // extern "C"
 
+namespace ww {
+
+// About how many primes are below b.
+static double primes_below(double b) { return b < 256.0 ? (b < 127.0 ? 0.0 : 54.0) : b / (log(b) - 1.1); }
+
+// Rows of the deep table worth their start-up in a segment of `numbers`
+// numbers below `high`: the primes below about B with B ln B = 7 times the
+// segment, since the primes near B spare 0.56 / (B ln B) of its numbers
+// their PRP test each (7 measured best on widths 1e6 to 2^28 among 3, 5, 7,
+// 10, 20, 33 and 60: 1e8 numbers in 687 us, at 33 in 843 us); and none above
+// the square root of `high`, whose multiples a smaller prime marks.  Any
+// count gives the same PRPs.
+int deep_rows_for(double numbers, u64 high) {
+    const double x = 7.0 * numbers;
+    double b = x / log(x / 10.0);
+    const double root = sqrt((double)high) + 1.0;
+    if (b > root) b = root;
+    const double n = primes_below(b) - 30.0;
+    return n < 0.0 ? 0 : n < (double)kDeepUse ? (int)n : kDeepUse;
+}
+
+}  // namespace ww
+
 namespace {
 
 // Resident CTAs of k_sieve_prp<G> on the current device (the dynamic
@@ -291,25 +314,6 @@ cudaError_t sieve_slots(int *slots) {
     *slots = sm_count() * (per_sm < 1 ? 1 : per_sm);
     if (keep) known[dev].store(*slots, std::memory_order_release);
     return cudaSuccess;
-}
-
-// About how many primes are below b.
-double primes_below(double b) { return b < 256.0 ? (b < 127.0 ? 0.0 : 54.0) : b / (log(b) - 1.1); }
-
-// Rows of the deep table worth their start-up in a segment of `numbers`
-// numbers below `high`: the primes below about B with B ln B = 7 times the
-// segment, since the primes near B spare 0.56 / (B ln B) of its numbers
-// their PRP test each (7 measured best on widths 1e6 to 2^28 among 3, 5, 7,
-// 10, 20, 33 and 60: 1e8 numbers in 687 us, at 33 in 843 us); and none above
-// the square root of `high`, whose multiples a smaller prime marks.  Any
-// count gives the same PRPs.
-int deep_rows_for(double numbers, uint64_t high) {
-    const double x = 7.0 * numbers;
-    double b = x / log(x / 10.0);
-    const double root = sqrt((double)high) + 1.0;
-    if (b > root) b = root;
-    const double n = primes_below(b) - 30.0;
-    return n < 0.0 ? 0 : n < (double)kDeepUse ? (int)n : kDeepUse;
 }
 
 template <class G>

@@ -135,6 +135,9 @@ __device__ __forceinline__ void step_hit(u32 &j0) {
 // The deep-sieve table lives once in device memory (ww_capi.cu); kernels
 // get its address as an argument.  Host code asks for it per device.
 const DeepRow *deep_rows_device();
+// How many of its rows to sieve a segment of `numbers` numbers below `high`
+// with (ww_capi.cu).
+int deep_rows_for(double numbers, u64 high);
 
 // Mark the odd multiples n = r*k of the first deep_n deep primes in the
 // segment, except those with k = 1 (mod ord_r(2)) (ww_deep.cuh says why).

@@ -80,7 +80,8 @@ __global__ void k_noalloc_finish(const NoAllocScratch *s, uint32_t n, ww_unit_re
         out[i].checksum = s->units[i].checksum;
         out[i].prp_count = s->units[i].prp_count;
         out[i].hits = s->units[i].hits;
-        out[i].tiles_done = s->units[i].tiles_done;
+        const u64 w = s->units[i].end - s->units[i].start;  // every tile is done: counted in full ones
+        out[i].tiles_done = (uint32_t)(w / NoAllocCfg::kTileNumbers + (w % NoAllocCfg::kTileNumbers ? 1 : 0));
     }
     const uint32_t nh = s->hit_count < kNoAllocMaxHits ? s->hit_count : kNoAllocMaxHits;
     for (uint32_t i = tid; i < nh && i < hit_cap; i += gridDim.x * blockDim.x) {
@@ -143,19 +144,24 @@ extern "C" int ww_batch_run_noalloc(const ww_unit *units, uint32_t n, ww_unit_re
     int rc = setup_device(dev, d);
     if (rc) return rc;
 
-    const u64 tile = NoAllocCfg::kTileNumbers;
-    u64 acc = 0;
+    double left = 0;  // numbers from unit i on
     for (uint32_t i = 0; i < n; ++i) {
         if (units[i].end < units[i].start || (units[i].end > units[i].start && units[i].start < 127)) {
             set_err("range %u: bad range [%llu, %llu)", i, (unsigned long long)units[i].start,
                     (unsigned long long)units[i].end);
             return WW_ERR_ARG;
         }
+        left += (double)(units[i].end - units[i].start);
+    }
+    u64 acc = 0;
+    for (uint32_t i = 0; i < n; ++i) {
         UnitState &u = g_h_units[i];
         memset(&u, 0, sizeof u);
         u.start = units[i].start;
         u.end = units[i].end;
-        const u64 w = units[i].end - units[i].start;
+        u.words = tile_words(left, d.grid, NoAllocCfg::kWords);
+        const u64 w = units[i].end - units[i].start, tile = 64ull * u.words;
+        left -= (double)w;
         u.n_tiles = w / tile + (w % tile ? 1 : 0);
         u.active = 1;
         g_h_first[i] = acc;
@@ -182,7 +188,8 @@ extern "C" int ww_batch_run_noalloc(const ww_unit *units, uint32_t n, ww_unit_re
     a.tile_first = s->tile_first;
     a.n_tiles = acc;
     a.next_tile = &s->next_tile;
-    a.epoch_tiles = &s->epoch;
+    a.epoch_words = &s->epoch;
+    for (int k = 0; k < kTileSizes; ++k) a.deep_n[k] = deep_rows_for(64.0 * (kTileMinWords << k), ~0ull);
     a.hit_p = s->hit_p;
     a.hit_result = s->hit_result;
     a.hit_rem = s->hit_rem;
