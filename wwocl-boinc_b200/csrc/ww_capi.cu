@@ -486,8 +486,9 @@ int ww_launch_test_prps(uint32_t *primecount, const uint64_t *g_prime, const uin
 int ww_launch_digits(const uint64_t *primes, uint64_t n, uint64_t *out, void *stream) {
     if (!primes || !out) return set_err("null pointer"), WW_ERR_ARG;
     if (n == 0) return WW_OK;
-    uint64_t blocks = (n + kTestThreads - 1) / kTestThreads;
-    if (blocks > (uint64_t)test_grid() * 8) blocks = (uint64_t)test_grid() * 8;
+    const uint64_t units = 2 * ((n + 31) / 32);  // one test of 32 primes a warp
+    uint64_t blocks = (units + kTestThreads / 32 - 1) / (kTestThreads / 32);
+    if (blocks > (uint64_t)test_grid()) blocks = (uint64_t)test_grid();
     k_digits<<<(unsigned)blocks, kTestThreads, 0, as_stream(stream)>>>((const u64 *)primes, n, (u64 *)out);
     WW_CHECK_LAUNCH();
     return WW_OK;

@@ -181,25 +181,27 @@ constexpr u64 kIdlePrime = 0xFFFFFFFFFFFFFFC5ull;  // 2^64 - 59
 template <class F>
 __device__ __forceinline__ void for_each_unit(u64 n, u64 *cursor, F &&f) {
     const int lane = threadIdx.x & 31;
-    u64 unit = (u64)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
-    const u64 stride = ((u64)gridDim.x * blockDim.x) >> 5;
-    const bool pull = cursor && n > stride;
+    // a list has below 2^37 primes, so units fit 32 bits (64-bit ones in this
+    // loop cost the test kernel 1 %)
+    const u32 m = (u32)n;
+    u32 unit = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    if (m <= (gridDim.x * blockDim.x) >> 5) cursor = nullptr;
     for (;;) {
-        if (pull) {
-            if (lane == 0) unit = atomicAdd((unsigned long long *)cursor, 1ull);
+        if (cursor) {
+            if (lane == 0) unit = (u32)atomicAdd((unsigned long long *)cursor, 1ull);
             unit = __shfl_sync(0xffffffffu, unit, 0);
         }
-        if (unit >= n) break;
+        if (unit >= m) break;
         f(unit);
-        unit += stride;
+        unit += (gridDim.x * blockDim.x) >> 5;
     }
 }
 
 // f(i, i < n) for 32 consecutive list indices a unit.
 template <class F>
 __device__ __forceinline__ void for_each_prime(u64 n, u64 *cursor, F &&f) {
-    for_each_unit((n + 31) / 32, cursor, [&](u64 unit) {
-        const u64 i = 32 * unit + (threadIdx.x & 31);
+    for_each_unit((n + 31) / 32, cursor, [&](u32 unit) {
+        const u64 i = 32ull * unit + (threadIdx.x & 31);
         f(i, i < n);
     });
 }
@@ -268,11 +270,11 @@ __global__ void __launch_bounds__(kTestThreads, WW_TEST_MINB) k_test_prps(u32 *p
                                                              u64 *totalprimecount, u64 capacity,
                                                              u64 *cursor) {
     const u64 n = min((u64)primecount[0], capacity);
-    const u64 groups = (n + 31) / 32;
+    const u32 groups = (u32)((n + 31) / 32);
     u64 sum = 0;
-    for_each_unit(2 * groups, cursor, [&](u64 unit) {
+    for_each_unit(2ull * groups, cursor, [&](u32 unit) {
         const bool wss = unit < groups;
-        const u64 i = 32 * (wss ? unit : unit - groups) + (threadIdx.x & 31);
+        const u64 i = 32ull * (wss ? unit : unit - groups) + (threadIdx.x & 31);
         const bool act = i < n;
         const u64 p = act ? prime[i] : kIdlePrime;
         const u64 q = act && inv ? inv[i] : inv64(p);
@@ -299,18 +301,20 @@ __global__ void __launch_bounds__(kTestThreads, WW_TEST_MINB) k_test_prps(u32 *p
     if (blockIdx.x == 0 && threadIdx.x == 0) count_update(primecount, totalprimecount);
 }
 
-__global__ void k_digits(const u64 *primes, u64 n, u64 *out) {
-    for_each_prime(n, nullptr, [&](u64 i, bool act) {
-        const u64 p = act ? primes[i] : kIdlePrime;
+// Units as in k_test_prps.
+__global__ void __launch_bounds__(kTestThreads, WW_TEST_MINB) k_digits(const u64 *primes, u64 n, u64 *out) {
+    const u32 groups = (u32)((n + 31) / 32);
+    for_each_unit(2ull * groups, nullptr, [&](u32 unit) {
+        const bool wss = unit < groups;
+        const u64 i = 32ull * (wss ? unit : unit - groups) + (threadIdx.x & 31);
+        const u64 p = i < n ? primes[i] : kIdlePrime;
         const u64 q = inv64(p);
         const D2 one = m2_one(p);
-        D2 s, c;
-        both_digits(p, q, one, s, c);
-        if (act) {
-            out[4 * i] = s.d0;
-            out[4 * i + 1] = s.d1;
-            out[4 * i + 2] = c.d0;
-            out[4 * i + 3] = c.d1;
+        const D2 d = wss ? wss_digits(p, q, one) : wieferich_digits(p, q, one);
+        if (i < n) {
+            u64 *to = out + 4 * i + (wss ? 2 : 0);
+            to[0] = d.d0;
+            to[1] = d.d1;
         }
     });
 }
