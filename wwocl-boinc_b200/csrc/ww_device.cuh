@@ -147,7 +147,11 @@ int deep_rows_for(double numbers, u64 high);
 // primes is marked by a whole warp (lane l takes the multiples l, l + 32,
 // ...; k then grows by 64 per step), the rest one prime per thread, so no
 // thread holds the others at the next barrier.
-constexpr int kDeepWarpPrimes = 512;
+constexpr int kDeepWarpPrimes = 1536;
+// Rows of the table the wide and narrow segments are sieved with: with 1 536
+// primes by warps, 2^30 numbers near 2^64 took 4.88 ms (35 000 rows 4.89, all
+// 81 995 with 1 024 by warps 4.96, and with 512 5.04).
+constexpr int kWideRows = kDeepUse < 50000 ? kDeepUse : 50000;
 
 __device__ __forceinline__ void deep_mark(u64 first, u32 nvalid, u32 *bitmap, int tid, int nthreads,
                                           const DeepRow *__restrict__ deep, int deep_n = kDeepUse,

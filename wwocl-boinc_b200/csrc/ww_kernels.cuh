@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(G::kThreads, WW_SIEVE_MINB_THREADS / G::kThrea
         // ---- deep sieve 113 < r < 2^WW_DEEP_BITS, sparing possible pseudoprimes
         const u64 nbase = b0 + seg_off + 1;
         deep_mark(nbase, (u32)nvalid, bitmap, threadIdx.x, G::kThreads, deep,
-                  G::kRuntime ? plan.deep_n : kDeepUse, G::kRuntime ? plan.warp_n : kDeepWarpPrimes);
+                  G::kRuntime ? plan.deep_n : kWideRows, G::kRuntime ? plan.warp_n : kDeepWarpPrimes);
         __syncthreads();
 
         // ---- warps take chunks of 32 words (or fewer) dynamically (so they reach the next
