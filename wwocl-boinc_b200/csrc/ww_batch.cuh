@@ -117,8 +117,9 @@ __device__ __forceinline__ void test_batch(const u64 *qp, const u32 *qu, int n_v
 #pragma unroll
     for (int k = 0; k < PPT; ++k) {
         const int idx = k * 32 + lane;
+        if (k * 32 >= n_valid) break;
         const bool act = idx < n_valid;
-        const u64 p = act ? qp[idx] : 0xFFFFFFFFFFFFFFC5ull;  // 2^64-59, a harmless prime
+        const u64 p = qp[act ? idx : 0];  // idle lanes repeat the first
         const u32 unit = act ? qu[idx] : 0u;
         const u64 q = inv64(p);
         const D2 one = m2_one(p);
@@ -143,7 +144,6 @@ __device__ __forceinline__ void test_batch(const u64 *qp, const u32 *qu, int n_v
         }
         // one atomic a batch when its PRPs are of one unit
         const u32 live = __ballot_sync(0xffffffffu, act);
-        if (live == 0) continue;
         const u32 unit0 = __shfl_sync(0xffffffffu, unit, __ffs((int)live) - 1);
         if (__all_sync(0xffffffffu, !act || unit == unit0)) {
             sum = warp_sum(sum);

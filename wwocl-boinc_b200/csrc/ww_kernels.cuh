@@ -167,9 +167,6 @@ __device__ __forceinline__ void count_update(u32 *primecount, u64 *totalprimecou
     if (pc > primecount[1]) primecount[1] = pc;
 }
 
-// A prime for the lanes past a list's end: the ladders run on whole warps.
-constexpr u64 kIdlePrime = 0xFFFFFFFFFFFFFFC5ull;  // 2^64 - 59
-
 // Runs f(unit) on whole warps for every unit < n.  With a work cursor (zeroed
 // before the launch) each warp pulls one unit at a time, so warps that run
 // ahead take more of the work and all finish together; without one (a
@@ -197,12 +194,14 @@ __device__ __forceinline__ void for_each_unit(u64 n, u64 *cursor, F &&f) {
     }
 }
 
-// f(i, i < n) for 32 consecutive list indices a unit.
+// f(i, whether the lane is one of the list's) for 32 consecutive list indices
+// a unit.  The ladders run on whole warps: lanes past the end repeat the last
+// prime, whose size is its neighbours'.
 template <class F>
 __device__ __forceinline__ void for_each_prime(u64 n, u64 *cursor, F &&f) {
     for_each_unit((n + 31) / 32, cursor, [&](u32 unit) {
         const u64 i = 32ull * unit + (threadIdx.x & 31);
-        f(i, i < n);
+        f(min(i, n - 1), i < n);
     });
 }
 
@@ -213,8 +212,8 @@ __global__ void __launch_bounds__(kTestThreads, WW_TEST_MINB) k_wieferich(u32 *p
     const u64 n = min((u64)primecount[0], capacity);
     u64 sum = 0;
     for_each_prime(n, cursor, [&](u64 i, bool act) {
-        const u64 p = act ? prime[i] : kIdlePrime;
-        const u64 q = act && inv ? inv[i] : inv64(p);
+        const u64 p = prime[i];
+        const u64 q = inv ? inv[i] : inv64(p);
         const D2 one = m2_one(p);
         if (act && g_one) {
             g_one[2 * i] = one.d0;
@@ -239,10 +238,10 @@ __global__ void __launch_bounds__(kTestThreads, WW_TEST_MINB) k_wallsunsun(const
     const u64 n = min((u64)primecount[0], capacity);
     u64 sum = 0;
     for_each_prime(n, cursor, [&](u64 i, bool act) {
-        const u64 p = act ? prime[i] : kIdlePrime;
-        const u64 q = act && inv ? inv[i] : inv64(p);
+        const u64 p = prime[i];
+        const u64 q = inv ? inv[i] : inv64(p);
         D2 one;
-        if (act && g_one) {
+        if (g_one) {
             one.d0 = g_one[2 * i];
             one.d1 = g_one[2 * i + 1];
         } else {
@@ -274,10 +273,11 @@ __global__ void __launch_bounds__(kTestThreads, WW_TEST_MINB) k_test_prps(u32 *p
     u64 sum = 0;
     for_each_unit(2ull * groups, cursor, [&](u32 unit) {
         const bool wss = unit < groups;
-        const u64 i = 32ull * (wss ? unit : unit - groups) + (threadIdx.x & 31);
-        const bool act = i < n;
-        const u64 p = act ? prime[i] : kIdlePrime;
-        const u64 q = act && inv ? inv[i] : inv64(p);
+        const u64 at = 32ull * (wss ? unit : unit - groups) + (threadIdx.x & 31);
+        const bool act = at < n;
+        const u64 i = min(at, n - 1);  // lanes past the end repeat the last prime
+        const u64 p = prime[i];
+        const u64 q = inv ? inv[i] : inv64(p);
         const D2 one = m2_one(p);
         int res = 1093, rem = 0, quot;
         u64 digit;
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kTestThreads, WW_TEST_MINB) k_digits(const u64
     for_each_unit(2ull * groups, nullptr, [&](u32 unit) {
         const bool wss = unit < groups;
         const u64 i = 32ull * (wss ? unit : unit - groups) + (threadIdx.x & 31);
-        const u64 p = i < n ? primes[i] : kIdlePrime;
+        const u64 p = primes[min(i, n - 1)];
         const u64 q = inv64(p);
         const D2 one = m2_one(p);
         const D2 d = wss ? wss_digits(p, q, one) : wieferich_digits(p, q, one);

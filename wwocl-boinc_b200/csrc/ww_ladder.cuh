@@ -269,13 +269,21 @@ WW_HD u64 power_windows(u64 e, int steps) {
 // The digit of the window at bit pos, below bit i (the top window is short).
 WW_HD u32 window_digit(u64 f, int pos, int i) { return (u32)(f >> pos) & ((1u << (i - pos)) - 1u); }
 
-#if defined(__CUDACC__)
 // A^2 / R mod n
-__device__ __forceinline__ u64 lz_sqr1(u64 a, const LzMod &m) {
+WW_HD u64 lz_sqr1(u64 a, const LzMod &m) {
     u64 u;
     u32 neg;
     return lz_low(lz_square(a), m, u, neg);
 }
+// A 2^(d - 32) mod n for 0 <= d < 32 (lz_shift's low digit)
+WW_HD u64 lz_shift1(u64 a, u32 d, const LzMod &m) {
+    const u32 w = ((u32)a << d) * (u32)m.q;
+    u32 neg;
+    const u64 r = lz_sub(a >> (32 - d), (u64)w * (u32)(m.p >> 32) + (((u64)w * (u32)m.p) >> 32), neg);
+    return lz_addp(r, neg, m);
+}
+
+#if defined(__CUDACC__)
 
 // The base-2 strong probable-prime test (sprp2) for a whole warp: all 32
 // lanes call it, and lanes with act false test the first active lane's number
@@ -307,16 +315,11 @@ __device__ __forceinline__ bool sprp2_warp(u64 n, bool act, u64 &q_out) {
     u64 a = one, unused;
     if (e0) a = mod_est(one >> (64 - e0), one << e0, n, 1.0 / (double)n, unused);
     int i = steps, pos = (steps + kWinBits - 1) / kWinBits * kWinBits;
-    const u32 n0 = (u32)n, n1 = (u32)(n >> 32);
     while (i > 0) {
         pos -= kWinBits;
         const u32 d = window_digit(f, pos, i);
         for (; i > pos; --i) a = lz_sqr1(a, m);
-        // a 2^(d-32): one 32-bit Montgomery step (lz_shift)
-        const u32 w = ((u32)a << d) * (u32)q;
-        u32 neg;
-        const u64 r = lz_sub(a >> (32 - d), (u64)w * n1 + (((u64)w * n0) >> 32), neg);
-        a = lz_addp(r, neg, m);
+        a = lz_shift1(a, d, m);
     }
     u64 ebits = nm1 << (63 - tw);  // bit tw at bit 63
     u64 at_t = 0;

@@ -168,11 +168,97 @@ WW_HD D2 lucas_finish(D2 e, D2 o, bool jodd, u64 p, u64 q) {
     return m2_div5(m2_redc(m2_sub(m2_dbl(d, p), a, p), p, q), p);
 }
 
+// For p < 2^32, p^2 fits a word: the same ladders on residues mod n = p^2 in
+// one-word Montgomery form, a third of the multiplies.  A whole warp takes it
+// or none of its lanes does (small_modulus); kept out of line, so that the
+// kernels' main loops keep their registers.
+WW_HD bool small_modulus(u64 p) {
+#if defined(__CUDA_ARCH__)
+    return __all_sync(0xffffffffu, (p >> 32) == 0);
+#else
+    return (p >> 32) == 0;
+#endif
+}
+
+#if defined(__CUDACC__)
+#define WW_HD_CALL static __host__ __device__ __noinline__
+#else
+#define WW_HD_CALL static inline
+#endif
+
+struct SmallMod {
+    LzMod m;     // n = p^2
+    u64 one;     // 2^64 mod n
+    double rn;   // 1 / (double)n
+};
+WW_HD SmallMod small_mod(u64 p) {
+    SmallMod s;
+    const u64 n = p * p;
+    s.m = lz_mod(n, inv64(n));
+    s.one = r_mod(n);
+    s.rn = 1.0 / (double)n;
+    return s;
+}
+// L R mod n for 1 <= L < 2^48
+WW_HD u64 small_times_r(u64 L, const SmallMod &s) {
+    u64 l, h, unused;
+    mul_wide(L, s.one, l, h);
+    return mod_est(h, l, s.m.p, s.rn, unused);
+}
+// (x R^-1 mod n) as digits by p
+WW_HD D2 small_digits(u64 x, u64 p, const SmallMod &s) {
+    D2 d;
+    d.d0 = mod_est(0, redc(x, 0, s.m.p, s.m.q), p, 1.0 / (double)p, d.d1);
+    return d;
+}
+
+WW_HD_CALL D2 wieferich_small(u64 p, int steps) {
+    const SmallMod s = small_mod(p);
+    const u64 f = power_windows(p >> 1, steps);
+    u64 a = small_times_r(1ull << (f >> steps), s);
+    int pos = (steps + kWinBits - 1) / kWinBits * kWinBits;
+    int i = steps;
+    while (i > 0) {
+        pos -= kWinBits;
+        const u32 d = window_digit(f, pos, i);
+        for (; i > pos; --i) a = lz_sqr1(a, s.m);
+        a = lz_shift1(a, d, s.m);
+    }
+    return small_digits(a, p, s);
+}
+
+WW_HD_CALL D2 wss_small(u64 p, u64 j, int steps) {
+    const SmallMod s = small_mod(p);
+    // R 2^32, squared: R^2; the constants -2 R^2 and -3 R^2
+    const u64 r2 = lz_sqr1(small_times_r(1ull << 32, s), s.m);
+    const u64 c2 = sub_mod(0, add_mod(r2, r2, s.m.p), s.m.p);
+    const u64 c3 = sub_mod(c2, r2, s.m.p);
+    const u32 k0 = (u32)(j >> steps);
+    bool kodd = k0 & 1u;
+    u64 e = small_times_r(lucas_even(k0 + (k0 & 1u)), s);
+    u64 o = small_times_r(lucas_even(k0 | 1u), s);
+    u64 jb = j << (63 - steps) << 1;
+    for (int i = steps; i > 0; --i) {
+        const bool bit = (long long)jb < 0;
+        jb <<= 1;
+        const u64 x = bit == kodd ? e : o;
+        u64 u;
+        u32 neg;
+        o = lz_low((u128)e * o + c3, s.m, u, neg);
+        e = lz_low(lz_square(x) + c2, s.m, u, neg);
+        kodd = bit;
+    }
+    const u64 a = kodd ? o : e, b = kodd ? e : o;  // W_j, W_j+1
+    const u64 d = sub_mod(b, a, s.m.p);
+    return m2_div5(small_digits(sub_mod(add_mod(d, d, s.m.p), a, s.m.p), p, s), p);
+}
+
 // 2^((p-1)/2) mod p^2 as canonical digits (wieferich.cl:219-245).
 WW_HD D2 wieferich_digits(u64 p, u64 q, D2 one) {
+    const int steps = ladder_steps(lucas_index(p));
+    if (small_modulus(p)) return wieferich_small(p, steps);
     const LzMod m = lz_mod(p, q);
     const double rp = 1.0 / (double)p;
-    const int steps = ladder_steps(lucas_index(p));
     const u64 f = power_windows(p >> 1, steps);
     D2 w = small_start(1ull << (f >> steps), one, p, rp);
     int pos = (steps + kWinBits - 1) / kWinBits * kWinBits;  // the window's low bit, once it is taken
@@ -196,10 +282,11 @@ WW_HD D2 wieferich_digits(u64 p, u64 q, D2 one) {
 
 // F_{p-(p|5)} mod p^2 as canonical digits (wallsunsun.cl:242-300).
 WW_HD D2 wss_digits(u64 p, u64 q, D2 one) {
-    const LzMod m = lz_mod(p, q);
-    const double rp = 1.0 / (double)p;
     const u64 j = lucas_index(p);
     const int steps = ladder_steps(j);
+    if (small_modulus(p)) return wss_small(p, j, steps);
+    const LzMod m = lz_mod(p, q);
+    const double rp = 1.0 / (double)p;
     const LadderConst c = ladder_const(one, m, rp);
     const u32 k0 = (u32)(j >> steps);
     bool kodd = k0 & 1u;
