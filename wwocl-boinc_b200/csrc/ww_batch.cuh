@@ -130,7 +130,7 @@ __device__ __forceinline__ void test_batch(const u64 *qp, const u32 *qu, int n_v
         if (JOINT) {
             both_digits(p, q, one, s, c);
         } else {
-            s = wieferich_digits(p, q, one);
+            s = wieferich_digits<false>(p, q, one);
             c = wss_digits(p, q, one);
         }
         u64 sum = 0;

@@ -17,13 +17,12 @@
 // any other integer instruction holds its pipe for 2, and the compiler
 // spreads moves and carries over both, so the time is about 3.15 cycles a
 // wide multiply and one for every other instruction, of which 87 % is
-// reached; occupancy (48 to 80 registers) moves it by 1 %.  A ladder step was
-// 319 instructions (54 wide multiplies) and is 235 (59) now.  Products are
-// unsigned __int128 ones: a 64x64->128 product is then 7.4 instructions and 16
-// cycles of the multiply pipe, against 11.5 and 24 for `a * b` beside
-// `__umul64hi(a, b)`, which share nothing.  Both tests over 2^24 primes of
-// [2^62, 2^64): 12.33 ms with canonical digits, a pair of squarings and
-// doublings bit by bit, 10.78 ms in this form (1 360 and 1 557 M primes/s).
+// reached; occupancy (48 to 80 registers) moves it by 1 %.  So what counts is
+// the number of instructions: a ladder step was 319 (54 wide multiplies) with
+// canonical digits, a pair of squarings and doublings bit by bit, 235 in this
+// form on __int128 products, and some 215 on the products below.  Both tests
+// over 2^24 primes of [2^62, 2^64): 12.33, 10.78 and 10.11 ms (1 360, 1 557 and
+// 1 660 M primes/s).
 #pragma once
 
 #include "ww_arith.cuh"
@@ -99,24 +98,106 @@ WW_HD u64 lz_sub(u64 a, u64 b, u32 &neg) {
 #endif
 }
 
-// a^2 from three 32x32 products: a0^2 + 2^64 a1^2 and a0 a1 shifted in by 33
-// bits.  One wide multiply fewer than a product of a by itself.
+// Products from four 32x32 ones (three for a square), each written so that
+// the cross products' sum is the addend of the top one, a1 b1 + (y:z) with the
+// carry of the word below: on the device a `mad.lo.cc` / `madc.hi.cc` pair on
+// the same factors is one wide multiply-add with carry in and out, so an
+// addend costs next to nothing.  A product is 6 instructions (7.4 as the
+// unsigned __int128 one, whose last word is added after the multiply), a
+// product plus a word 8 (11.4).  Over 2^24 primes: 10.78 ms with __int128
+// products and added constants, 10.67 with the square's constant as its
+// addend, 10.33 with the cross products', 10.11 ms in this form throughout.
+WW_HD u128 lz_mul(u64 a, u64 b) {
+#if defined(__CUDA_ARCH__)
+    u64 lo, hi;
+    asm("{\n\t.reg .u64 e, o;\n\t.reg .u32 r0, r1, r2, r3, x, y, z;\n\t"
+        "mul.wide.u32 o, %2, %5;\n\t"
+        "mov.b64 {x, y}, o;\n\t"
+        "mad.lo.cc.u32 x, %3, %4, x;\n\t"
+        "madc.hi.cc.u32 y, %3, %4, y;\n\t"
+        "addc.u32 z, 0, 0;\n\t"
+        "mul.wide.u32 e, %2, %4;\n\t"
+        "mov.b64 {r0, r1}, e;\n\t"
+        "add.cc.u32 r1, r1, x;\n\t"
+        "madc.lo.cc.u32 r2, %3, %5, y;\n\t"
+        "madc.hi.u32 r3, %3, %5, z;\n\t"
+        "mov.b64 %0, {r0, r1};\n\t"
+        "mov.b64 %1, {r2, r3};\n\t}"
+        : "=l"(lo), "=l"(hi)
+        : "r"((u32)a), "r"((u32)(a >> 32)), "r"((u32)b), "r"((u32)(b >> 32)));
+    return ((u128)hi << 64) | lo;
+#else
+    return (u128)a * b;
+#endif
+}
+
+// The high word.
+WW_HD u64 lz_hi(u64 a, u64 b) {
+#if defined(__CUDA_ARCH__)
+    u64 hi;
+    asm("{\n\t.reg .u64 e, o;\n\t.reg .u32 r0, r1, r2, r3, x, y, z;\n\t"
+        "mul.wide.u32 o, %1, %4;\n\t"
+        "mov.b64 {x, y}, o;\n\t"
+        "mad.lo.cc.u32 x, %2, %3, x;\n\t"
+        "madc.hi.cc.u32 y, %2, %3, y;\n\t"
+        "addc.u32 z, 0, 0;\n\t"
+        "mul.wide.u32 e, %1, %3;\n\t"
+        "mov.b64 {r0, r1}, e;\n\t"
+        "add.cc.u32 r1, r1, x;\n\t"
+        "madc.lo.cc.u32 r2, %2, %4, y;\n\t"
+        "madc.hi.u32 r3, %2, %4, z;\n\t"
+        "mov.b64 %0, {r2, r3};\n\t}"
+        : "=l"(hi)
+        : "r"((u32)a), "r"((u32)(a >> 32)), "r"((u32)b), "r"((u32)(b >> 32)));
+    return hi;
+#else
+    return mul_hi(a, b);
+#endif
+}
+
+// a b + k
+WW_HD u128 lz_mad(u64 a, u64 b, u64 k) {
+#if defined(__CUDA_ARCH__)
+    u64 lo, hi;
+    asm("{\n\t.reg .u64 o;\n\t.reg .u32 r0, r1, r2, r3, x, y, z, kl, kh;\n\t"
+        "mov.b64 {kl, kh}, %6;\n\t"
+        "mul.wide.u32 o, %2, %5;\n\t"
+        "mov.b64 {x, y}, o;\n\t"
+        "mad.lo.cc.u32 x, %3, %4, x;\n\t"
+        "madc.hi.cc.u32 y, %3, %4, y;\n\t"
+        "addc.u32 z, 0, 0;\n\t"
+        "mad.lo.cc.u32 r0, %2, %4, kl;\n\t"
+        "madc.hi.cc.u32 r1, %2, %4, kh;\n\t"
+        "addc.cc.u32 y, y, 0;\n\t"
+        "addc.u32 z, z, 0;\n\t"
+        "add.cc.u32 r1, r1, x;\n\t"
+        "madc.lo.cc.u32 r2, %3, %5, y;\n\t"
+        "madc.hi.u32 r3, %3, %5, z;\n\t"
+        "mov.b64 %0, {r0, r1};\n\t"
+        "mov.b64 %1, {r2, r3};\n\t}"
+        : "=l"(lo), "=l"(hi)
+        : "r"((u32)a), "r"((u32)(a >> 32)), "r"((u32)b), "r"((u32)(b >> 32)), "l"(k));
+    return ((u128)hi << 64) | lo;
+#else
+    return (u128)a * b + k;
+#endif
+}
+
+// a^2: a0 a1 is shifted in by 33 bits.
 WW_HD u128 lz_square(u64 a) {
 #if defined(__CUDA_ARCH__)
     u64 lo, hi;
-    asm("{\n\t.reg .u64 e, f, o;\n\t.reg .u32 r0, r1, r2, r3, x, y, z;\n\t"
-        "mul.wide.u32 e, %2, %2;\n\t"
+    asm("{\n\t.reg .u64 e, o;\n\t.reg .u32 r0, r1, r2, r3, x, y, z;\n\t"
         "mul.wide.u32 o, %2, %3;\n\t"
-        "mul.wide.u32 f, %3, %3;\n\t"
-        "mov.b64 {r0, r1}, e;\n\t"
-        "mov.b64 {r2, r3}, f;\n\t"
         "mov.b64 {x, y}, o;\n\t"
         "shf.l.clamp.b32 z, x, y, 1;\n\t"
         "shl.b32 x, x, 1;\n\t"
         "shr.u32 y, y, 31;\n\t"
+        "mul.wide.u32 e, %2, %2;\n\t"
+        "mov.b64 {r0, r1}, e;\n\t"
         "add.cc.u32 r1, r1, x;\n\t"
-        "addc.cc.u32 r2, r2, z;\n\t"
-        "addc.u32 r3, r3, y;\n\t"
+        "madc.lo.cc.u32 r2, %3, %3, z;\n\t"
+        "madc.hi.u32 r3, %3, %3, y;\n\t"
         "mov.b64 %0, {r0, r1};\n\t"
         "mov.b64 %1, {r2, r3};\n\t}"
         : "=l"(lo), "=l"(hi) : "r"((u32)a), "r"((u32)(a >> 32)));
@@ -126,17 +207,44 @@ WW_HD u128 lz_square(u64 a) {
 #endif
 }
 
+// a^2 + k0 (below 2^128 for a^2 + k0 of the ladders: a < p, k0 < p)
+WW_HD u128 lz_square_add(u64 a, u64 k0) {
+#if defined(__CUDA_ARCH__)
+    u64 lo, hi;
+    asm("{\n\t.reg .u64 o;\n\t.reg .u32 r0, r1, r2, r3, x, y, z, kl, kh;\n\t"
+        "mov.b64 {kl, kh}, %4;\n\t"
+        "mul.wide.u32 o, %2, %3;\n\t"
+        "mov.b64 {x, y}, o;\n\t"
+        "shf.l.clamp.b32 z, x, y, 1;\n\t"
+        "shl.b32 x, x, 1;\n\t"
+        "shr.u32 y, y, 31;\n\t"
+        "mad.lo.cc.u32 r0, %2, %2, kl;\n\t"
+        "madc.hi.cc.u32 r1, %2, %2, kh;\n\t"
+        "addc.cc.u32 z, z, 0;\n\t"
+        "addc.u32 y, y, 0;\n\t"
+        "add.cc.u32 r1, r1, x;\n\t"
+        "madc.lo.cc.u32 r2, %3, %3, z;\n\t"
+        "madc.hi.u32 r3, %3, %3, y;\n\t"
+        "mov.b64 %0, {r0, r1};\n\t"
+        "mov.b64 %1, {r2, r3};\n\t}"
+        : "=l"(lo), "=l"(hi) : "r"((u32)a), "r"((u32)(a >> 32)), "l"(k0));
+    return ((u128)hi << 64) | lo;
+#else
+    return (u128)a * a + k0;
+#endif
+}
+
 // Low digit of T / R for T < p 2^64: the digit, u = T q mod 2^64 and the
 // borrow mask that the high digit takes over.
 WW_HD u64 lz_low(u128 T, const LzMod &m, u64 &u, u32 &neg) {
     u = (u64)T * m.q;
-    const u64 r = lz_sub((u64)(T >> 64), mul_hi(u, m.p), neg);
+    const u64 r = lz_sub((u64)(T >> 64), lz_hi(u, m.p), neg);
     return lz_addp(r, neg, m);
 }
 
 // High digit from the sum (k:h:s), k signed: ((k:h) - hi(s q p)) in [-p, 2p).
 WW_HD u64 lz_high(u64 s, u64 h, u32 k, const LzMod &m) {
-    const u64 v = mul_hi(s * m.q, m.p);
+    const u64 v = lz_hi(s * m.q, m.p);
 #if defined(__CUDA_ARCH__)
     u64 r;
     u32 t;
@@ -150,35 +258,25 @@ WW_HD u64 lz_high(u64 s, u64 h, u32 k, const LzMod &m) {
 #endif
 }
 
-// (k:h:s) = a + b + u + k1 + 2^64 neg, neg a borrow mask (0 or -1).
-WW_HD void lz_sum(u128 a, u128 b, u64 u, u64 k1, u32 neg, u64 &s, u64 &h, u32 &k) {
+// As lz_high for the sum (k:h:s) less 2^64 for the borrow mask neg.
+WW_HD u64 lz_high_less(u64 s, u64 h, u32 k, u32 neg, const LzMod &m) {
 #if defined(__CUDA_ARCH__)
-    u64 neg2;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(neg2) : "r"(neg));
-    asm("add.cc.u64 %0, %3, %5;\n\t"
-        "addc.cc.u64 %1, %4, %6;\n\t"
-        "addc.u32 %2, 0, %9;\n\t"
-        "add.cc.u64 %0, %0, %7;\n\t"
-        "addc.cc.u64 %1, %1, 0;\n\t"
-        "addc.u32 %2, %2, 0;\n\t"
-        "add.cc.u64 %0, %0, %8;\n\t"
-        "addc.cc.u64 %1, %1, %10;\n\t"
-        "addc.u32 %2, %2, 0;"
-        : "=&l"(s), "=&l"(h), "=&r"(k)
-        : "l"((u64)a), "l"((u64)(a >> 64)), "l"((u64)b), "l"((u64)(b >> 64)), "l"(u), "l"(k1), "r"(neg), "l"(neg2));
+    const u64 v = lz_hi(s * m.q, m.p);
+    u64 r;
+    u32 t;
+    asm("{\n\t.reg .u32 z;\n\t"
+        "sub.cc.u32 z, 0, %5;\n\t"
+        "subc.cc.u64 %0, %2, %3;\n\t"
+        "subc.u32 %1, %4, 0;\n\t}"
+        : "=&l"(r), "=r"(t) : "l"(h), "l"(v), "r"(k), "r"(neg));
+    return lz_fix(r, t, m);
 #else
-    u128 t = a + b;
-    k = t < a;
-    t += u;
-    k += t < u;
-    t += k1;
-    k += t < k1;
-    s = (u64)t;
-    h = (u64)(t >> 64);
     if (neg) k -= h-- == 0;
+    return lz_high(s, h, k, m);
 #endif
 }
-// the same without k1
+
+// (k:h:s) = a + b + u + 2^64 neg, neg a borrow mask (0 or -1).
 WW_HD void lz_sum(u128 a, u128 b, u64 u, u32 neg, u64 &s, u64 &h, u32 &k) {
 #if defined(__CUDA_ARCH__)
     u64 neg2;
@@ -192,7 +290,13 @@ WW_HD void lz_sum(u128 a, u128 b, u64 u, u32 neg, u64 &s, u64 &h, u32 &k) {
         : "=&l"(s), "=&l"(h), "=&r"(k)
         : "l"((u64)a), "l"((u64)(a >> 64)), "l"((u64)b), "l"((u64)(b >> 64)), "l"(u), "r"(neg), "l"(neg2));
 #else
-    lz_sum(a, b, u, 0, neg, s, h, k);
+    u128 t = a + b;
+    k = t < a;
+    t += u;
+    k += t < u;
+    s = (u64)t;
+    h = (u64)(t >> 64);
+    if (neg) k -= h-- == 0;
 #endif
 }
 
@@ -202,30 +306,49 @@ WW_HD D2 lz_sqr(D2 x, const LzMod &m) {
     u32 neg, k;
     D2 r;
     r.d0 = lz_low(lz_square(x.d0), m, u, neg);
-    const u128 c = (u128)x.d0 * x.d1;
+    const u128 c = lz_mul(x.d0, x.d1);
     lz_sum(c, c, u, neg, s, h, k);
     r.d1 = lz_high(s, h, k, m);
     return r;
 }
-// (X^2 + K) / R, K canonical
-WW_HD D2 lz_sqr_add(D2 x, D2 kk, const LzMod &m) {
+// (X^2 + K) / R for K = kh.d0 + 2 p kh.d1, both digits below p (lz_halve)
+WW_HD D2 lz_sqr_add(D2 x, D2 kh, const LzMod &m) {
     u64 u, s, h;
     u32 neg, k;
     D2 r;
-    r.d0 = lz_low(lz_square(x.d0) + kk.d0, m, u, neg);
-    const u128 c = (u128)x.d0 * x.d1;
-    lz_sum(c, c, u, kk.d1, neg, s, h, k);
+    r.d0 = lz_low(lz_square_add(x.d0, kh.d0), m, u, neg);
+    const u128 c = lz_mad(x.d0, x.d1, kh.d1);
+    lz_sum(c, c, u, neg, s, h, k);
     r.d1 = lz_high(s, h, k, m);
     return r;
+}
+// Canonical K as lz_sqr_add takes it: its high digit halved mod p
+WW_HD D2 lz_halve(D2 kk, u64 p) {
+    const u64 add = (kk.d1 & 1) ? p : 0;
+    const u64 sum = kk.d1 + add;
+    kk.d1 = (sum >> 1) | ((u64)(sum < add) << 63);
+    return kk;
 }
 // (X Y + K) / R, K canonical
 WW_HD D2 lz_mul_add(D2 x, D2 y, D2 kk, const LzMod &m) {
     u64 u, s, h;
     u32 neg, k;
     D2 r;
-    r.d0 = lz_low((u128)x.d0 * y.d0 + kk.d0, m, u, neg);
-    lz_sum((u128)x.d0 * y.d1, (u128)x.d1 * y.d0, u, kk.d1, neg, s, h, k);
-    r.d1 = lz_high(s, h, k, m);
+    r.d0 = lz_low(lz_mad(x.d0, y.d0, kk.d0), m, u, neg);
+    const u128 a = lz_mad(x.d0, y.d1, u), b = lz_mad(x.d1, y.d0, kk.d1);
+#if defined(__CUDA_ARCH__)
+    asm("add.cc.u64 %0, %3, %5;\n\t"
+        "addc.cc.u64 %1, %4, %6;\n\t"
+        "addc.u32 %2, 0, 0;"
+        : "=&l"(s), "=&l"(h), "=&r"(k)
+        : "l"((u64)a), "l"((u64)(a >> 64)), "l"((u64)b), "l"((u64)(b >> 64)));
+#else
+    const u128 t = a + b;
+    k = t < a;
+    s = (u64)t;
+    h = (u64)(t >> 64);
+#endif
+    r.d1 = lz_high_less(s, h, k, neg, m);
     return r;
 }
 

@@ -132,7 +132,7 @@ WW_HD D2 small_start(u64 L, D2 one, u64 p, double rp) {
 }
 
 struct LadderConst {
-    D2 m2, m3;  // -2 R^2 and -3 R^2
+    D2 m2h, m3;  // -2 R^2 (as lz_halve leaves it) and -3 R^2
 };
 WW_HD LadderConst ladder_const(D2 one, const LzMod &m, double rp) {
     // R 2^32, squared: R^2 2^64 / R = R^2
@@ -140,8 +140,9 @@ WW_HD LadderConst ladder_const(D2 one, const LzMod &m, double rp) {
     const D2 zero = {0, 0};
     const D2 t2 = m2_dbl(r2, m.p);
     LadderConst c;
-    c.m2 = m2_sub(zero, t2, m.p);
-    c.m3 = m2_sub(c.m2, r2, m.p);
+    const D2 m2 = m2_sub(zero, t2, m.p);
+    c.m2h = lz_halve(m2, m.p);
+    c.m3 = m2_sub(m2, r2, m.p);
     return c;
 }
 
@@ -155,7 +156,7 @@ WW_HD LadderConst ladder_const(D2 one, const LzMod &m, double rp) {
 WW_HD void lucas_step(D2 &e, D2 &o, bool &kodd, bool bit, const LadderConst &c, const LzMod &m) {
     const D2 s = sel(bit == kodd, e, o);
     o = lz_mul_add(e, o, c.m3, m);
-    e = lz_sqr_add(s, c.m2, m);
+    e = lz_sqr_add(s, c.m2h, m);
     kodd = bit;
 }
 
@@ -244,8 +245,8 @@ WW_HD_CALL D2 wss_small(u64 p, u64 j, int steps) {
         const u64 x = bit == kodd ? e : o;
         u64 u;
         u32 neg;
-        o = lz_low((u128)e * o + c3, s.m, u, neg);
-        e = lz_low(lz_square(x) + c2, s.m, u, neg);
+        o = lz_low(lz_mad(e, o, c3), s.m, u, neg);
+        e = lz_low(lz_square_add(x, c2), s.m, u, neg);
         kodd = bit;
     }
     const u64 a = kodd ? o : e, b = kodd ? e : o;  // W_j, W_j+1
@@ -253,7 +254,12 @@ WW_HD_CALL D2 wss_small(u64 p, u64 j, int steps) {
     return m2_div5(small_digits(sub_mod(add_mod(d, d, s.m.p), a, s.m.p), p, s), p);
 }
 
-// 2^((p-1)/2) mod p^2 as canonical digits (wieferich.cl:219-245).
+// 2^((p-1)/2) mod p^2 as canonical digits (wieferich.cl:219-245).  The five
+// squarings of a window are written out for the list kernels (1 658 M
+// primes/s, as a loop 1 635) and a loop (kWriteOut false) in the tile engine,
+// whose warps run sieve, PRP test and both ladders at the same time and were
+// waiting for instructions (96 ranges: 42.2 ms written out, 40.3 as a loop).
+template <bool kWriteOut = true>
 WW_HD D2 wieferich_digits(u64 p, u64 q, D2 one) {
     const int steps = ladder_steps(lucas_index(p));
     if (small_modulus(p)) return wieferich_small(p, steps);
@@ -266,7 +272,7 @@ WW_HD D2 wieferich_digits(u64 p, u64 q, D2 one) {
     while (i > 0) {
         pos -= kWinBits;
         const u32 d = window_digit(f, pos, i);
-        if (i - pos == kWinBits) {  // written out: 1 543 against 1 536 M primes/s
+        if (kWriteOut && i - pos == kWinBits) {
             w = lz_sqr(w, m);
             w = lz_sqr(w, m);
             w = lz_sqr(w, m);
@@ -274,6 +280,9 @@ WW_HD D2 wieferich_digits(u64 p, u64 q, D2 one) {
             w = lz_sqr(w, m);
             i = pos;
         }
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
         for (; i > pos; --i) w = lz_sqr(w, m);
         w = lz_shift(w, d, m);
     }
