@@ -145,3 +145,20 @@ def test_gpu_cut_tiles_equal_units_alone(ww, widths, cfg):
         assert [(r["checksum"], r["prp_count"], r["hits"]) for r in done] == want
         assert [r["prps_stored"] for r in done] == [w[1] for w in want]
         server.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cfg", [(16384, 512, 1, 1), (8192, 256, 1, 1)])
+@pytest.mark.parametrize("low", [127, 2**32 - 300_000, 2**32 + 1])
+def test_gpu_joint_loop_around_one_word_primes(ww, cfg, low):
+    """Both tests in one loop on whole warps of primes below 2^32, on warps
+    that hold some of each, and above: each unit as alone on the plain path,
+    where the tests run one after the other."""
+    units = [(low, low + 600_000), (low + 600_000, low + 600_100), (2**40 + low, 2**40 + low + 50_000)]
+    with ww.Context(0, max_prps=100_000) as ctx:
+        batch = ww.Batch(ctx)
+        batch.set_config(*cfg)
+        got = batch.run(units)
+        alone = [ctx.run_range(a, b) for a, b in units]
+    assert [(r["checksum"], r["prp_count"], r["hits"]) for r in got] == [
+        (r["checksum"], r["total_prp_count"], r["result_count"]) for r in alone]
