@@ -21,20 +21,22 @@
 // two-digit sum and difference, the finish of a two-digit product) are PTX
 // borrow chains: each turns its borrow into a mask m (0 or 2^32 - 1) and
 // adds m & p back, instead of a compare and a select.  -DWW_NO_PTX_CC selects
-// the C forms (measured 3 % slower on the fused test kernel).
+// the C forms (measured 3 % slower on a fused test kernel built on them).
+// The ladders' own corrections and products are in ww_ladder.cuh; what is
+// here starts and ends them, and is what they are tested against.
 #if !defined(WW_NO_PTX_CC) && !defined(WW_PTX_CC)
 #define WW_PTX_CC 1
 #endif
 //
 // With every correction on the integer ALU, that pipe was the busier of the
-// two integer pipes in the test loops (73 % against 71 %: adds, borrows,
-// selects and shifts outnumber the multiplies), so the "& p" of a correction
-// runs as two 32-bit multiplies by the mask on the multiply pipe instead
-// (add_masked, form 2), which leaves the multiply pipe the busier one.  WW_MAD_SITES picks where:
+// two integer pipes in test loops built on these operations (73 % against
+// 71 %: adds, borrows, selects and shifts outnumber the multiplies), so the
+// "& p" of a correction runs as two 32-bit multiplies by the mask on the
+// multiply pipe instead (add_masked, form 2).  WW_MAD_SITES picks where:
 // bit 0 the mod-n REDC and sum of the PRP test, bit 1 the finish of a
 // two-digit product, bit 2 two-digit differences, bit 3 two-digit sums; the
-// places left out keep the ALU form.  Measured on a B200 (fused test kernel,
-// 2^26 primes, before the three-product square): sites 1-3 in form 2,
+// places left out keep the ALU form.  Measured on a B200 (a fused test kernel
+// on these operations, 2^26 primes, before the three-product square): sites 1-3 in form 2,
 // 1 318 M primes/s; sites 1-2, 1 340 M (with the square); sites 1 and 3 or
 // 2 and 3, 1 283 and 1 216 M; the ALU mask form everywhere, 1 233 M; the
 // compare/select sums and and+add masks before it, 1 148 M; form 1 (one wide
@@ -84,11 +86,7 @@ WW_HD void mul_wide(u64 a, u64 b, u64 &lo, u64 &hi) {
 }
 
 // a^2 as (hi:lo) from three 32x32 products (a0^2, a1^2 and a0 a1 once):
-// a^2 = a0^2 + 2^33 a0 a1 + 2^64 a1^2.  Used for the low digit of a
-// two-digit square, where it measured 3.5 % faster on the fused test kernel
-// than the four-product mul_wide; in the PRP test's squaring and as the
-// high word of a REDC's u*p (three products, with the carry of the known
-// low word) it measured slower.
+// a^2 = a0^2 + 2^33 a0 a1 + 2^64 a1^2.  The low digit of m2_sqr.
 WW_HD void sqr_wide(u64 a, u64 &lo, u64 &hi) {
     const u32 a0 = (u32)a, a1 = (u32)(a >> 32);
     const u64 m = (u64)a0 * a1;

@@ -297,22 +297,23 @@ int deep_rows_for(double numbers, u64 high) {
 namespace {
 
 // Resident CTAs of k_sieve_prp<G> on the current device (the dynamic
-// shared memory limit is raised first; asked of the driver once per device).
+// shared memory limit is raised first; the count is asked of the driver once
+// per device).
 template <class G>
 cudaError_t sieve_slots(int *slots) {
     static std::atomic<int> known[kCursorPoolDevices];
+    cudaError_t e = cudaFuncSetAttribute(k_sieve_prp<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::kSmem);
+    if (e != cudaSuccess) return e;
     int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     const bool keep = dev >= 0 && dev < kCursorPoolDevices;
-    if (keep && (*slots = known[dev].load(std::memory_order_acquire)) > 0) return cudaSuccess;
-    e = cudaFuncSetAttribute(k_sieve_prp<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::kSmem);
-    if (e != cudaSuccess) return e;
+    if (keep && (*slots = known[dev].load(std::memory_order_relaxed)) > 0) return cudaSuccess;
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_sieve_prp<G>, G::kThreads, G::kSmem);
     if (e != cudaSuccess) return e;
     *slots = sm_count() * (per_sm < 1 ? 1 : per_sm);
-    if (keep) known[dev].store(*slots, std::memory_order_release);
+    if (keep) known[dev].store(*slots, std::memory_order_relaxed);
     return cudaSuccess;
 }
 

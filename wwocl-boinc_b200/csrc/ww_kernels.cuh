@@ -25,7 +25,8 @@ namespace ww {
 // Threads per SM the sieve's launch bounds ask for: 1024 holds it to 64
 // registers (2 CTAs of 512, or 4 of 256, per SM).  Uncapped it takes 128;
 // at 512 or 768 (1 CTA of 512 per SM, 128 registers) the sieve measured
-// 7.19 against 5.90 ms per 2^30 numbers on a B200.
+// 7.19 against 5.90 ms per 2^30 numbers on a B200 (with a doubling per bit
+// in the PRP test; 4.87 ms with its windows).
 #ifndef WW_SIEVE_MINB_THREADS
 #define WW_SIEVE_MINB_THREADS 1024
 #endif
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(kTestThreads, WW_TEST_MINB) k_wallsunsun(const
 // Wieferich ones, so the last of a launch are short, and a list shorter than
 // the grid's warps runs its two tests on different warps.  The two in one
 // loop (both_digits, 78 registers) measured 1 509 against 1 543 M primes/s
-// on 2^24 primes.
+// on 2^24 primes (with the products as __int128 multiplies; 1 660 M since).
 __global__ void __launch_bounds__(kTestThreads, WW_TEST_MINB) k_test_prps(u32 *primecount, const u64 *prime,
                                                              const u64 *inv, HitOut hits, u64 *checksum,
                                                              u64 *totalprimecount, u64 capacity,
