@@ -87,21 +87,21 @@ def algorithmic_imad_per_prime(primes: np.ndarray) -> tuple[float, float]:
     """32-bit multiply instructions per prime, counted with fixed costs: a
     64x64->128 product = 8, a low 64-bit product = 4, a high 64-bit product =
     8, so a two-digit square mod p^2 = 40 and a product = 48 (38 for the
-    square k_test_prps runs, whose low digit is squared from three 32x32
+    squares k_test_prps runs, whose low digit is squared from three 32x32
     products instead of four).  k = bitlength(p).
 
     Returns (reference_count, executed_count):
       reference_count: the reference kernels' algorithm -- Wieferich k-3
         squarings (wieferich.cl:196-328), the Lucas ladder k-1 steps of two
         squarings and one product (wallsunsun.cl:221-354): 40(k-3) + 128(k-1).
-      executed_count: what k_test_prps runs -- both ladders start from the
-        top bits of their exponents (three small numbers turned into
-        Montgomery form, 40 each), then Wieferich k-6 squarings and the Lucas
-        ladder k-6 steps of two squarings (38 each), two conversions out of
-        Montgomery form (24 each): 114(k-6) + 120 + 48."""
+      executed_count: what k_test_prps runs -- k-6 steps each: a Wieferich
+        squaring with a fifth of a five-bit window (two one-word reductions,
+        10), and a Lucas step of a squaring and a product; four starts of 12,
+        the square of 2^64 and two conversions out of Montgomery form (24
+        each): 126(k-6) + 134."""
     bits = np.floor(np.log2(primes.astype(np.float64))) + 1  # exact away from powers of two
     ref = 40.0 * (bits - 3) + 128.0 * (bits - 1)
-    run = 114.0 * (bits - 6) + 168.0
+    run = 126.0 * (bits - 6) + 134.0
     return float(ref.mean()), float(run.mean())
 
 
@@ -265,14 +265,15 @@ def run_range_pipeline(ww, local: int, width: int, ckpt: int = 1 << 30, chain_pe
         # end to end over sieve + tests, in the same 32-bit multiply units as
         # the test kernel's roofline (k = 64 here): the reference's SPRP of a
         # candidate is 20(k-1) and its sieve hands ~5.3 candidates per PRP to
-        # it; here the SPRP starts after the top five bits of n-1 (20(k-5)
-        # plus a 12-multiply start) and the deep sieve to 2^depth leaves
+        # it; here the SPRP starts after the top five bits of n-1, squares from
+        # three products and takes five bits a window (19(k-6) plus a start of
+        # 20), and the deep sieve to 2^depth leaves
         # 0.5615 / ln 2^depth candidates per integer, against the PRP density
         # 1 / ln 2^64
         k = 64
         ref_ops = 40.0 * (k - 3) + 128.0 * (k - 1) + 5.3 * 20.0 * (k - 1)
         cand = (0.5615 / np.log(2.0**depth)) * np.log(2.0**64)
-        run_ops = 114.0 * (k - 6) + 168.0 + cand * (20.0 * (k - 5) + 12.0)
+        run_ops = 126.0 * (k - 6) + 134.0 + cand * (19.0 * (k - 6) + 20.0)
         rate = out["primes_per_s"]
         out["roofline_end_to_end"] = {
             "peak_tops": chain_peak / 1e12,
@@ -285,8 +286,8 @@ def run_range_pipeline(ww, local: int, width: int, ckpt: int = 1 << 30, chain_pe
         # depth as above; the sieving itself is shifts, ORs and atomics)
         seg = out["segment_2p30"]
         cand_per_number = cand / np.log(2.0**64)
-        sieve_ops = cand_per_number * (20.0 * (k - 5) + 12.0) * min(width, ckpt)
-        out["sieve_roofline"] = {"executed_ops_per_number": cand_per_number * (20.0 * (k - 5) + 12.0),
+        sieve_ops = cand_per_number * (19.0 * (k - 6) + 20.0) * min(width, ckpt)
+        out["sieve_roofline"] = {"executed_ops_per_number": cand_per_number * (19.0 * (k - 6) + 20.0),
                                  "achieved_tops": sieve_ops / (seg["sieve_ms"] * 1e-3) / 1e12,
                                  "frac_chain_peak": sieve_ops / (seg["sieve_ms"] * 1e-3) / chain_peak,
                                  "note": "candidates per number estimated as 0.5615 / ln 2^depth (Mertens)"}
@@ -649,7 +650,7 @@ def main():
                              "it can pass 1.0; executed.frac is the pipe-occupancy view",
                 "executed": {"ops_per_prime": per_prime_run, "achieved": achieved_run / 1e12,
                              "frac": achieved_run / chain_peak,
-                             "note": "multiplies k_test_prps itself runs: 114(k-6) + 168 (ladders started from their top bits, three-product squares of the low digit)"},
+                             "note": "multiplies k_test_prps itself runs: 126(k-6) + 134 (ladders started from their top bits, three-product squares of the low digit)"},
                 "mad_lo_only": {"peak": madlo_peak / 1e12, "frac": achieved / madlo_peak,
                                 "frac_executed": achieved_run / madlo_peak},
                 "hbm": {"bytes_per_launch": 16 * n, "GBps": 16 * n / (launch_ms * 1e-3) / 1e9,
@@ -699,7 +700,8 @@ def main():
                     "d2h_bytes_per_step": 32 + hit_bytes * hits_per_step,
                     "call": "ww_test_prps_host (pinned list, copy of chunk k+1 overlapping the test of chunk k) "
                             "+ ww_read_counters", "checksum_equal": bool(e2e_checksum == checksum)},
-            "gpu_launches": args.steps, "roofline": roofline, "cpu_baseline": cpu,
+            "gpu_launches": 2 * args.steps,  # a step: k_clear_results and k_test_prps
+            "roofline": roofline, "cpu_baseline": cpu,
             "clocks": clocks.summary(), "checksum": "%016X" % checksum, "list_gen_s": gen_s}
     # last key: every leg's results in a few hundred bytes (kept by a reader
     # that keeps only the end of the output)
