@@ -278,7 +278,7 @@ int ww_batch_tune(ww_ctx *ctx, const ww_unit *sample, uint32_t n, ww_batch_cfg *
  * memory up front and forbid later allocations, or latency-bound loops
  * that cannot afford an allocation's device-wide synchronisation, get the
  * same per-range results as ww_batch_run without any allocation: the
- * scratch lives in one fixed __device__ array of the library (480 KiB per
+ * scratch lives in one fixed __device__ array of the library (448 KiB per
  * device, kept until exit).  units: host array, n <= 4096 ranges;
  * out[n], hits[hit_cap] (at most 4096 records), hit_unit[hit_cap] (may be
  * NULL) and *hit_count are device memory; work is queued on `stream` (a
@@ -298,8 +298,8 @@ int ww_batch_run_noalloc(const ww_unit *units, uint32_t n, ww_unit_result *out, 
  * per process).  Continuous batching: requests wait in a host queue and are
  * admitted into device slots while slots and PRP-buffer memory last (each
  * request reserves ww_prp_count_bound(start, end) * 8 bytes); every
- * ww_server_step runs one bounded launch of the tile engine over all
- * admitted requests (round-robin, each request's sieve cursor, checksum,
+ * ww_server_step runs one bounded launch of the tile engine over the
+ * admitted requests (earliest deadline first, each request's checksum,
  * counters and PRP buffer resident on the device) and returns the requests
  * that finished.  A request's results equal those of running it alone.
  * ------------------------------------------------------------------------- */
@@ -320,9 +320,12 @@ typedef struct {
 typedef struct {
     uint64_t prp_pool_bytes; /* device memory for per-request PRP buffers */
     uint32_t max_active;     /* device slots */
-    uint32_t epoch_tiles;    /* tiles one step launches (rounded to whole
-                                waves of resident CTAs when above one wave;
-                                0: one wave) */
+    uint32_t epoch_tiles;    /* full tiles (64 * seg_words numbers) whose numbers
+                                one step hands out (rounded to whole waves of
+                                one 512-thread tile per SM when above one wave;
+                                0: one wave).  A request's tiles may be smaller:
+                                a step takes as many as have those numbers, and
+                                less than one tile more */
     uint32_t max_hits;       /* hit records per step */
     uint32_t store_prps;     /* 1: keep each request's PRP list on the device */
 } ww_server_cfg;

@@ -197,3 +197,41 @@ def test_requests_admitted_mid_flight_equal_alone_and_oracle(ww, ctx, oracle):
         assert np.array_equal(np.sort(prps), wprps), rid
         assert hits == sorted(whits), rid
     assert got[4998][0]["hits"] >= 1 and got[4999][0]["hits"] >= 1
+
+
+def test_a_step_hands_out_what_was_asked(ww, ctx):
+    """epoch_tiles = 2: a step takes the numbers of two full tiles and less
+    than one tile (here at most 2^18 numbers) more, also while a request in
+    small tiles and one in large ones are at hand, where every resident CTA
+    looks for a tile at once.  Counted by the steps that all the work needs."""
+    small, wide = 9_000_000, 160_000_000
+    srv = ww.Server(ctx, prp_pool_bytes=1 << 28, max_active=4, epoch_tiles=2)
+    srv.submit([(1, 10**15, 10**15 + small)])  # alone: cut into the smallest tiles
+    done, steps = {r["id"]: r for r in srv.step()}, 1
+    srv.submit([(2, 10**16, 10**16 + wide)])
+    while len(done) < 2 and steps < 1000:
+        done.update({r["id"]: r for r in srv.step()})
+        steps += 1
+    srv.close()
+    assert (small + wide) / (2**21 + 2**18) <= steps <= (small + wide) / 2**21 + 2
+    for rid, a, w in ((1, 10**15, small), (2, 10**16, wide)):
+        ref = ctx.run_range(a, a + w)
+        assert (done[rid]["checksum"], done[rid]["prp_count"]) == (ref["checksum"], ref["total_prp_count"])
+
+
+def test_finished_requests_wait_for_room_to_be_reported(ww, ctx):
+    """A step whose caller has room for fewer results than requests finished
+    reports the rest at the next steps, which have no tiles left to run."""
+    reqs = [(i, 10**14 + 10**6 * i, 10**14 + 10**6 * i + 100_000) for i in range(5)]
+    srv = ww.Server(ctx, prp_pool_bytes=1 << 26, max_active=8)
+    srv.submit(reqs)
+    buf, n, seen = (ww.RequestResult * 1)(), C.c_uint32(0), []
+    for _ in range(len(reqs)):
+        ww.check(ww.lib().ww_server_step(ctx.h, buf, 1, C.byref(n)), "ww_server_step")
+        assert n.value == 1
+        seen.append((buf[0].id, buf[0].checksum, buf[0].prp_count))
+    assert srv.status()[:2] == (0, 0)
+    srv.close()
+    for rid, a, b in reqs:
+        ref = ctx.run_range(a, b)
+        assert (rid, ref["checksum"], ref["total_prp_count"]) in seen

@@ -107,7 +107,6 @@ struct BatchState {
     UnitState *d_units = nullptr;
     u64 *d_first = nullptr;
     u64 *d_next = nullptr;
-    u32 *d_epoch = nullptr;
     u32 *d_hit_count = nullptr, *d_overflow = nullptr, *d_hit_unit = nullptr;
     u64 *d_hit_p = nullptr;
     int *d_hit_res = nullptr, *d_hit_rem = nullptr, *d_hit_quot = nullptr;
@@ -124,7 +123,6 @@ struct BatchState {
         cudaFree(d_units);
         cudaFree(d_first);
         cudaFree(d_next);
-        cudaFree(d_epoch);
         cudaFree(d_hit_count);
         cudaFree(d_overflow);
         cudaFree(d_hit_unit);
@@ -163,7 +161,6 @@ int ensure_capacity(BatchState &b, u32 n_units, u32 hit_cap) {
     }
     // each on its own, so a call after a failed one allocates what is missing
     if (!b.d_next) WW_CU(cudaMalloc(&b.d_next, sizeof(u64)));
-    if (!b.d_epoch) WW_CU(cudaMalloc(&b.d_epoch, sizeof(u32)));
     if (!b.d_hit_count) WW_CU(cudaMalloc(&b.d_hit_count, sizeof(u32)));
     if (!b.d_overflow) WW_CU(cudaMalloc(&b.d_overflow, sizeof(u32)));
     if (hit_cap > b.hit_cap) {
@@ -201,8 +198,8 @@ BatchArgs make_args(BatchState &b, u32 n, u64 n_tiles) {
     a.tile_first = b.d_first;
     a.n_tiles = n_tiles;
     a.next_tile = b.d_next;
-    a.epoch_words = b.d_epoch;
-    a.budget = 0;
+    a.shares = nullptr;
+    a.n_shares = 0;
     a.hit_p = b.d_hit_p;
     a.hit_result = b.d_hit_res;
     a.hit_rem = b.d_hit_rem;
@@ -476,6 +473,7 @@ struct ServerSlot {
     ww_request r{};
     double t_submit = 0, t_admit = 0;
     u64 pool_off = 0, pool_len = 0;  // bytes
+    u64 next_tile = 0;               // sieve cursor: next tile to hand out
 };
 
 struct ServerState {
@@ -485,9 +483,9 @@ struct ServerState {
     int step_tiles = 0;        // full tiles' worth of words a step hands out
     UnitState *d_slots = nullptr, *h_slots = nullptr;
     u64 *pool = nullptr;
-    u32 *d_epoch = nullptr, *d_hit_count = nullptr, *d_overflow = nullptr;
-    u32 *d_order = nullptr, *h_order = nullptr;  // slots in deadline order (pinned mirror)
-    double tile_s = 0;                           // EMA of a step's seconds per wave of tiles
+    u32 *d_hit_count = nullptr, *d_overflow = nullptr;
+    StepShare *d_shares = nullptr, *h_shares = nullptr;  // a step's tiles in deadline order (pinned mirror)
+    double tile_s = 0;                                   // EMA of a step's seconds per wave of tiles
     u32 *d_hit_unit = nullptr, *h_hit_unit = nullptr;
     u64 *d_hit_p = nullptr, *h_hit_p = nullptr;
     int *d_hit_res = nullptr, *d_hit_rem = nullptr, *d_hit_quot = nullptr;
@@ -503,8 +501,7 @@ struct ServerState {
     ~ServerState() {
         cudaFree(d_slots);
         cudaFree(pool);
-        cudaFree(d_epoch);
-        cudaFree(d_order);
+        cudaFree(d_shares);
         cudaFree(d_hit_count);
         cudaFree(d_overflow);
         cudaFree(d_hit_unit);
@@ -519,7 +516,7 @@ struct ServerState {
         if (h_hit_rem) cudaFreeHost(h_hit_rem);
         if (h_hit_quot) cudaFreeHost(h_hit_quot);
         if (h_counts) cudaFreeHost(h_counts);
-        if (h_order) cudaFreeHost(h_order);
+        if (h_shares) cudaFreeHost(h_shares);
     }
 
     // first fit over the coalesced free list
@@ -624,9 +621,8 @@ int server_init(ServerState &s, ww_ctx *ctx, const ww_server_cfg *cfg) {
         WW_CU(cudaMalloc(&s.pool, cfg->prp_pool_bytes));
         s.free_blocks[0] = cfg->prp_pool_bytes & ~7ull;
     }
-    WW_CU(cudaMalloc(&s.d_order, (size_t)n * 4));
-    WW_CU(cudaMallocHost(&s.h_order, (size_t)n * 4));
-    WW_CU(cudaMalloc(&s.d_epoch, 4));
+    WW_CU(cudaMalloc(&s.d_shares, (size_t)n * sizeof(StepShare)));
+    WW_CU(cudaMallocHost(&s.h_shares, (size_t)n * sizeof(StepShare)));
     WW_CU(cudaMalloc(&s.d_hit_count, 4));
     WW_CU(cudaMalloc(&s.d_overflow, 4));
     WW_CU(cudaMalloc(&s.d_hit_unit, (size_t)h * 4));
@@ -709,7 +705,7 @@ int ww_server_step(ww_ctx *ctx, ww_request_result *done, uint32_t cap, uint32_t 
         for (u32 k = 0; k < n; ++k)
             if (s.slots[k].busy) {
                 const UnitState &u = s.h_slots[k];
-                left += 64.0 * u.words * (double)(u.n_tiles - std::min(u.next_tile, u.n_tiles));
+                left += 64.0 * u.words * (double)(u.n_tiles - s.slots[k].next_tile);
             }
         for (const ServerReq &q : s.queue) left += (double)(q.r.end - q.r.start);
     }
@@ -730,6 +726,7 @@ int ww_server_step(ww_ctx *ctx, ww_request_result *done, uint32_t cap, uint32_t 
         sl.t_admit = mono_s();
         sl.pool_off = off;
         sl.pool_len = len;
+        sl.next_tile = 0;
         UnitState &u = s.h_slots[k];
         memset(&u, 0, sizeof u);
         u.start = q.r.start;
@@ -758,7 +755,6 @@ int ww_server_step(ww_ctx *ctx, ww_request_result *done, uint32_t cap, uint32_t 
     // p50.  Until a step has been timed, the order is that of submission.
     const double wave_s = s.tile_s > 0 ? s.tile_s : 1e-6;
     const double wave_words = (double)std::max(1, s.step_tiles) * s.e->seg_words;
-    u32 n_order = 0;
     std::vector<std::pair<double, u32>> by_deadline;
     by_deadline.reserve(active);
     for (u32 k = 0; k < n; ++k)
@@ -766,26 +762,37 @@ int ww_server_step(ww_ctx *ctx, ww_request_result *done, uint32_t cap, uint32_t 
             by_deadline.emplace_back(s.slots[k].t_submit +
                                          2.0 * (double)s.h_slots[k].n_tiles * s.h_slots[k].words / wave_words * wave_s, k);
     std::sort(by_deadline.begin(), by_deadline.end());
-    for (const auto &d : by_deadline) s.h_order[n_order++] = d.second;
+    // the step's tiles: in that order, until they have the words of the full
+    // tiles asked for (the last unit's share rounded up to its tiles).  Whole
+    // waves of the step's tiles: a partial last wave would leave most SMs idle
+    // while its few tiles finish
+    const u64 g = (u64)s.step_tiles, asked = s.cfg.epoch_tiles;
+    const u64 tiles = asked == 0 ? g : asked < g ? asked : std::max<u64>(1, (asked + g / 2) / g) * g;
+    u64 room = tiles * (u64)s.e->seg_words, step_words = 0, step_tiles = 0;
+    u32 n_shares = 0;
+    for (const auto &d : by_deadline) {
+        const u32 k = d.second;
+        const u64 from = s.slots[k].next_tile, words = s.h_slots[k].words;
+        const u64 take = std::min(s.h_slots[k].n_tiles - from, (room + words - 1) / words);
+        if (!take) continue;
+        s.h_shares[n_shares++] = StepShare{from, from + take, k, 0};
+        step_tiles += take;
+        step_words += take * words;
+        room -= std::min(room, take * words);
+    }
     if (changed)
         WW_CU(cudaMemcpyAsync(s.d_slots, s.h_slots, (size_t)n * sizeof(UnitState), cudaMemcpyHostToDevice, st));
-    WW_CU(cudaMemcpyAsync(s.d_order, s.h_order, (size_t)n_order * 4, cudaMemcpyHostToDevice, st));
-    WW_CU(cudaMemsetAsync(s.d_epoch, 0, 4, st));
+    if (n_shares)
+        WW_CU(cudaMemcpyAsync(s.d_shares, s.h_shares, (size_t)n_shares * sizeof(StepShare), cudaMemcpyHostToDevice, st));
     WW_CU(cudaMemsetAsync(s.d_hit_count, 0, 4, st));
     WW_CU(cudaMemsetAsync(s.d_overflow, 0, 4, st));
     BatchArgs a;
     memset(&a, 0, sizeof a);
     a.units = s.d_slots;
     a.n_units = n;
-    a.order = s.d_order;
-    a.n_order = n_order;
-    a.epoch_words = s.d_epoch;
+    a.shares = s.d_shares;
+    a.n_shares = n_shares;
     fill_deep_n(a);
-    // whole waves of the step's tiles: a partial last wave would leave most
-    // SMs idle while its few tiles finish
-    const u64 g = (u64)s.step_tiles, asked = s.cfg.epoch_tiles;
-    const u64 tiles = asked == 0 ? g : asked < g ? asked : std::max<u64>(1, (asked + g / 2) / g) * g;
-    a.budget = (u32)std::min<u64>(tiles * (u64)s.e->seg_words, 0xf0000000ull);
     a.hit_p = s.d_hit_p;
     a.hit_result = s.d_hit_res;
     a.hit_rem = s.d_hit_rem;
@@ -796,31 +803,20 @@ int ww_server_step(ww_ctx *ctx, ww_request_result *done, uint32_t cap, uint32_t 
     a.overflow = s.d_overflow;
     a.deep = deep_rows_device();
     if (!a.deep) return WW_ERR_CUDA;
-    u32 least = (u32)s.e->seg_words;  // no more CTAs than the budget has tiles
-    for (u32 k = 0; k < n; ++k)
-        if (s.slots[k].busy) least = std::min(least, s.h_slots[k].words);
-    const int grid = (int)std::min<u64>((u64)s.grid, std::max<u32>(1, a.budget / least));
-    u64 words_before = 0;
-    for (u32 k = 0; k < n; ++k)
-        if (s.slots[k].busy)
-            words_before += std::min(s.h_slots[k].next_tile, s.h_slots[k].n_tiles) * s.h_slots[k].words;
     const double t_launch = mono_s();
-    s.e->serve_kernel<<<grid, s.e->threads, s.e->smem, st>>>(a);
-    WW_CU(cudaGetLastError());
+    if (n_shares) {  // none when every request at hand is done and waits to be reported
+        const int grid = (int)std::min<u64>((u64)s.grid, step_tiles);
+        s.e->serve_kernel<<<grid, s.e->threads, s.e->smem, st>>>(a);
+        WW_CU(cudaGetLastError());
+        for (u32 i = 0; i < n_shares; ++i) s.slots[s.h_shares[i].unit].next_tile = s.h_shares[i].end;
+    }
     WW_CU(cudaMemcpyAsync(s.h_slots, s.d_slots, (size_t)n * sizeof(UnitState), cudaMemcpyDeviceToHost, st));
     WW_CU(cudaMemcpyAsync(s.h_counts, s.d_hit_count, 4, cudaMemcpyDeviceToHost, st));
     WW_CU(cudaMemcpyAsync(s.h_counts + 1, s.d_overflow, 4, cudaMemcpyDeviceToHost, st));
     WW_CU(cudaStreamSynchronize(st));
-    {  // seconds per wave of tiles, from this step's words and time
-        u64 words_after = 0;
-        for (u32 k = 0; k < n; ++k)
-            if (s.slots[k].busy)
-                words_after += std::min(s.h_slots[k].next_tile, s.h_slots[k].n_tiles) * s.h_slots[k].words;
-        const u64 ran = words_after - words_before;
-        if (ran) {
-            const double per = (mono_s() - t_launch) / std::ceil((double)ran / wave_words);
-            s.tile_s = s.tile_s > 0 ? 0.8 * s.tile_s + 0.2 * per : per;
-        }
+    if (step_words) {  // seconds per wave of tiles, from this step's words and time
+        const double per = (mono_s() - t_launch) / std::ceil((double)step_words / wave_words);
+        s.tile_s = s.tile_s > 0 ? 0.8 * s.tile_s + 0.2 * per : per;
     }
     const u32 nh = std::min(s.h_counts[0], s.cfg.max_hits);
     if (nh) {

@@ -29,7 +29,6 @@ namespace ww {
 struct UnitState {
     u64 start, end;          // [start, end), start >= 127 unless empty
     u64 n_tiles;             // ceil((end - start) / tile)
-    u64 next_tile;           // sieve cursor: next tile to hand out (serving)
     u64 checksum;            // sum of both checksum terms
     u64 prp_count;           // PRPs tested
     u64 *prp_out;            // optional PRP buffer of the range (nullptr: none)
@@ -44,6 +43,12 @@ struct UnitState {
 constexpr int kTileMinWords = 128;
 constexpr int kTileSizes = 9;
 
+// Serving: the tiles [next, end) of one unit that a launch hands out.
+struct StepShare {
+    u64 next, end;
+    u32 unit, pad;
+};
+
 struct BatchArgs {
     UnitState *units;
     u32 n_units;
@@ -51,14 +56,10 @@ struct BatchArgs {
     const u64 *tile_first;
     u64 n_tiles;
     u64 *next_tile;          // queue head
-    // serving: tiles of about `budget` words in all this launch, handed out in
-    // the order of `order` (slot indices, earliest deadline first; n_order
-    // entries)
-    u32 *epoch_words;
-    u32 budget;
-    const u32 *order;
-    u32 n_order;
-    // hits: p, result, rem, quot, unit
+    // serving: this launch's tiles, n_shares units in the order they go out
+    // (earliest deadline first)
+    StepShare *shares;
+    u32 n_shares;
     u64 *hit_p;
     int *hit_result, *hit_rem, *hit_quot;
     u32 *hit_unit;
@@ -178,10 +179,11 @@ constexpr size_t batch_smem_bytes() {
 }
 
 // Hand out the next tile.  Batch: the global queue head over the static
-// tile table.  Serving: the first unit in the host's priority order that
-// has tiles left, through that unit's own cursor, until the tiles handed out
-// this launch have `budget` words; the loop is bounded by the number of
-// units, so an exhausted queue ends the kernel instead of spinning.
+// tile table.  Serving: the first of the launch's shares with tiles left,
+// through that share's own cursor.  The host cuts the shares to the step's
+// size, so a step hands out exactly those tiles, whichever CTAs come first;
+// the loop is bounded by the number of shares, so an exhausted step ends the
+// kernel instead of spinning.
 template <bool SERVE>
 __device__ __forceinline__ bool next_tile(const BatchArgs &a, u32 &unit, u64 &tile) {
     if constexpr (!SERVE) {
@@ -196,19 +198,14 @@ __device__ __forceinline__ bool next_tile(const BatchArgs &a, u32 &unit, u64 &ti
         tile = t - a.tile_first[lo];
         return true;
     } else {
-        // a tile counts when it is taken, not when it is looked for: CTAs that
-        // race for a unit's last tile would use up the budget
-        if (*(volatile u32 *)a.epoch_words >= a.budget) return false;
-        for (u32 i = 0; i < a.n_order; ++i) {
-            const u32 k = a.order[i];
-            UnitState &u = a.units[k];
+        for (u32 i = 0; i < a.n_shares; ++i) {
+            StepShare &sh = a.shares[i];
             // the cursor is read past L1 (other CTAs move it); a stale value
-            // only costs an atomic that finds the unit exhausted
-            if (!u.active || *(volatile u64 *)&u.next_tile >= u.n_tiles) continue;
-            const u64 t = atomicAdd((unsigned long long *)&u.next_tile, 1ull);
-            if (t < u.n_tiles) {
-                atomicAdd(a.epoch_words, u.words);
-                unit = k;
+            // only costs an atomic that finds the share exhausted
+            if (*(volatile u64 *)&sh.next >= sh.end) continue;
+            const u64 t = atomicAdd((unsigned long long *)&sh.next, 1ull);
+            if (t < sh.end) {
+                unit = sh.unit;
                 tile = t;
                 return true;
             }
