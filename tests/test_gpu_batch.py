@@ -119,3 +119,28 @@ def test_hit_overflow_keeps_results(ww, ctx, oracle):
         # a batch whose hits fit clears the flag
         b.run([(10**15, 10**15 + 10**6)])
         assert not b.hit_overflow
+
+
+def test_every_configuration_is_near_the_fastest(ww):
+    """No compiled configuration is a trap: on a mix large enough to fill the
+    GPU each takes less than twice the fastest one's time (they lie within a
+    factor of 1.35; four and eight primes per thread once took two and three
+    times as long), with the same results."""
+    import time
+
+    units = ww.uneven_units(7, 24, wmin=1e6, wmax=1e8)
+    times, results = {}, set()
+    with ww.Context(0, max_prps=1 << 12) as ctx:
+        batch = ww.Batch(ctx)
+        for cfg in ww.batch_configs():
+            batch.set_config(*cfg)
+            best = float("inf")
+            for _ in range(3):
+                t = time.perf_counter()
+                got = batch.run(units)
+                best = min(best, time.perf_counter() - t)
+            times[cfg] = best
+            results.add(tuple((r["checksum"], r["prp_count"], r["hits"]) for r in got))
+    assert len(results) == 1
+    fastest = min(times.values())
+    assert {c: round(t / fastest, 2) for c, t in times.items() if t >= 2 * fastest} == {}

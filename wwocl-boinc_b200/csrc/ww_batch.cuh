@@ -115,7 +115,11 @@ __device__ __forceinline__ void emit_batch_hit(const BatchArgs &a, u32 unit, u64
 template <int PPT, bool JOINT>
 __device__ __forceinline__ void test_batch(const u64 *qp, const u32 *qu, int n_valid, const BatchArgs &a) {
     const int lane = threadIdx.x & 31;
-#pragma unroll
+    // one copy of the ladders: written out PPT times, warps at different
+    // places of them waited for instructions (96 ranges of 1e6 to 1e8 numbers
+    // with 2, 4 and 8 primes per thread in 2^19-number tiles 49.3, 84.3 and
+    // 126.6 ms, as a loop 41.3, 43.0 and 43.4; with one 41.1)
+#pragma unroll 1
     for (int k = 0; k < PPT; ++k) {
         const int idx = k * 32 + lane;
         if (k * 32 >= n_valid) break;
