@@ -700,7 +700,7 @@ def main():
                     "d2h_bytes_per_step": 32 + hit_bytes * hits_per_step,
                     "call": "ww_test_prps_host (pinned list, copy of chunk k+1 overlapping the test of chunk k) "
                             "+ ww_read_counters", "checksum_equal": bool(e2e_checksum == checksum)},
-            "gpu_launches": 2 * args.steps,  # a step: k_clear_results and k_test_prps
+            "gpu_launches": args.steps,  # k_test_prps once a step
             "roofline": roofline, "cpu_baseline": cpu,
             "clocks": clocks.summary(), "checksum": "%016X" % checksum, "list_gen_s": gen_s}
     # last key: every leg's results in a few hundred bytes (kept by a reader

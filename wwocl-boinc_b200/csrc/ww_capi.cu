@@ -502,24 +502,16 @@ int ww_launch_digits(const uint64_t *primes, uint64_t n, uint64_t *out, void *st
 
 namespace {
 
+// primecount[0], the segment's count, comes first: ww_clear_results zeroes the rest.
 struct DevCounters {
+    unsigned int primecount[2];
     unsigned long long checksum;
     unsigned long long total;
     unsigned int resultcount;
-    unsigned int primecount[2];
     unsigned int overflow;
 };
 
 __global__ void k_set_count(unsigned int *pc, unsigned int v) { pc[0] = v; }
-
-// ww_clear_results in one launch: everything but the segment's count
-__global__ void k_clear_results(DevCounters *c) {
-    c->checksum = 0;
-    c->total = 0;
-    c->resultcount = 0;
-    c->primecount[1] = 0;
-    c->overflow = 0;
-}
 
 }  // namespace
 
@@ -724,8 +716,10 @@ int ww_get_buffers(ww_ctx *c, ww_buffers *b) {
 
 int ww_clear_results(ww_ctx *c) {
     if (!c) return set_err("null ctx"), WW_ERR_ARG;
-    k_clear_results<<<1, 1, 0, c->stream>>>(c->dc);
-    WW_CHECK_LAUNCH();
+    // one memset, which (unlike a kernel launch) is taken whatever the calling
+    // thread's current device is
+    constexpr size_t kept = sizeof(unsigned int);
+    WW_CU(cudaMemsetAsync((char *)c->dc + kept, 0, sizeof(DevCounters) - kept, c->stream));
     return WW_OK;
 }
 
