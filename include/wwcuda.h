@@ -401,19 +401,35 @@ int ww_count_prps(ww_ctx *ctx, uint64_t lo, uint64_t hi, uint64_t *count);
 int ww_selftest_digits(const uint64_t *primes, uint64_t n, uint64_t *out);
 int ww_selftest_range(uint64_t lo, uint64_t hi, uint64_t *prp_count, uint64_t *checksum,
                       uint32_t *result_count);
-/* One operation of the kernels' mod p^2 arithmetic on the host, for
- * checking it operand by operand: op & 15 = 0 X*Y/2^64, 1 X^2/2^64,
- * 2 X/2^64 (mod p^2); op >> 4 picks the formulation (0 the kernels' own,
+/* One operation of the canonical mod p^2 arithmetic on the host (what starts
+ * and ends the ladders; their steps are ww_selftest_ladder's), for checking
+ * it operand by operand: op & 15 = 0 X*Y/2^64, 1 X^2/2^64,
+ * 2 X/2^64 (mod p^2); op >> 4 picks the formulation (0 the build's own,
  * 1 64-bit products, 2 PTX carry chains, 3 wide 32x32+64 products).
  * Inputs and outputs are digit pairs x0 + p x1; xy = (x0, x1, y0, y1) per
  * case, out = (z0, z1). */
 int ww_selftest_m2(int op, uint64_t p, const uint64_t *xy, uint64_t n, uint64_t *out);
-/* The same check on the device, through the instruction sequences the
- * kernels run (borrow masks, multiply-pipe corrections): op 0-2 as above,
+/* The same check on the device (borrow masks, multiply-pipe corrections):
+ * op 0-2 as above,
  * 3 X+Y, 4 X-Y, 5 2X (mod p^2), and on the low digits alone 6 x0*y0/2^64,
  * 7 x0+y0, 8 (x1 2^64 + x0)/2^64 (mod p).  Host arrays; synchronises and
  * allocates its own device copy (no reference counterpart: a test hook). */
 int ww_devtest_m2(int device, int op, uint64_t p, const uint64_t *xy, uint64_t n, uint64_t *out);
+/* One operation of the ladders' own arithmetic for an odd modulus p, on the
+ * host (its C forms) and on the device (the instruction sequences that the
+ * test and PRP kernels run).  in = (x0, x1, y0, y1, k0, k1) per case, out =
+ * three words (unused ones zero); R = 2^64, digits X = x0 + p x1 with x0 < p
+ * and x1 below 2p and 2^64 (K canonical), results likewise:
+ *   0 X^2/R   1 (X^2 + K)/R   2 (X Y + K)/R   3 X 2^(d-32)  (mod p^2),
+ *   4 x0^2/R  5 x0 2^(d-32)   6 (x0 y0 + k0)/R  7 (x0^2 + k0)/R  (mod p),
+ *   with d = k0 & 31 and all operands of 4-7 below p;
+ * the whole products of any words
+ *   8 x0 y0  9 its high word  10 x0 y0 + k0  11 x0^2  12 x0^2 + k0;
+ *   13 (x1:x0) + (y1:y0) + k0 - 2^64 (k1 & 1) as three words, the top signed;
+ * and the high digit of a sum (y0:x1:x0), y0 signed, that the reduction takes
+ * to [-p, 2p): 14 as it is, 15 less 2^64 (k1 & 1). */
+int ww_selftest_ladder(int op, uint64_t p, const uint64_t *in, uint64_t n, uint64_t *out);
+int ww_devtest_ladder(int device, int op, uint64_t p, const uint64_t *in, uint64_t n, uint64_t *out);
 /* The kernels' PRP-test candidates of [lo, hi) computed on the host
  * (small primes 3..113, then the deep sieve, which leaves unmarked every
  * multiple r*k with k = 1 (mod ord_r(2)): r itself and every possible

@@ -1,10 +1,10 @@
-"""Operand-level parity of the device arithmetic: every operation the test and
-sieve kernels are built from (two-digit products, squares, the exit from
+"""Operand-level parity of the canonical device arithmetic, which starts and
+ends the test kernels' ladders (two-digit products, squares, the exit from
 Montgomery form, sums and differences mod p^2, and the mod-p Montgomery
-product, sum and reduction of the PRP test), run on the GPU through the same
-inline-PTX sequences the kernels execute, against exact integer arithmetic,
+product, sum and reduction), run on the GPU against exact integer arithmetic,
 including the digits 0, 1, p-1 and moduli at the 2^32, 2^62, 2^63 and 2^64
-edges."""
+edges.  The steps of the ladders and of the PRP test are in
+test_ladder_operands.py."""
 import numpy as np
 import pytest
 

@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/wwcuda.h"
+#include "ww_ladder_case.cuh"
 #include "ww_tests.cuh"
 
 using namespace ww;
@@ -211,7 +212,7 @@ int ww_selftest_range(uint64_t lo, uint64_t hi, uint64_t *prp_count, uint64_t *c
                            59u, 61u, 67u, 71u, 73u, 79u, 83u, 89u, 97u, 101u, 103u, 107u, 109u, 113u})
             small |= (n % r == 0);
         u64 q = 0;
-        if (small || !prp_test(n, q)) continue;  // the kernels' SPRP loop
+        if (small || !prp_test(n, q)) continue;  // bit by bit; the kernels take windows (sprp2_warp)
         const D2 one = m2_one(n);
         const D2 s = wieferich_digits(n, q, one);
         const D2 c = wss_digits(n, q, one);
@@ -228,7 +229,7 @@ int ww_selftest_range(uint64_t lo, uint64_t hi, uint64_t *prp_count, uint64_t *c
 }  // extern "C"
 
 // ---------------------------------------------------------------------------
-// Operation-level check of the two-digit arithmetic the kernels run (host
+// Operation-level check of the canonical two-digit arithmetic (host
 // instantiation of the same source): op 0 product, 1 square, 2 leave
 // Montgomery form.  xy holds (x0, x1, y0, y1) per case, out (z0, z1).
 
@@ -257,6 +258,13 @@ extern "C" int ww_selftest_m2(int op, uint64_t p, const uint64_t *xy, uint64_t n
         case 3: m2_cases<ArithWide>(op, p, xy, n, out); break;
         default: m2_cases<WW_ARITH>(op, p, xy, n, out); break;
     }
+    return WW_OK;
+}
+
+extern "C" int ww_selftest_ladder(int op, uint64_t p, const uint64_t *in, uint64_t n, uint64_t *out) {
+    if ((p & 1) == 0 || p < 3 || ((!in || !out) && n) || op < 0 || op >= kLadderOps) return WW_ERR_ARG;
+    const LzMod m = lz_mod(p, inv64(p));
+    for (uint64_t i = 0; i < n; ++i) ladder_case(op, m, (const u64 *)in + 6 * i, (u64 *)out + 3 * i);
     return WW_OK;
 }
 

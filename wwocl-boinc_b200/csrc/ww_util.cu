@@ -10,6 +10,7 @@
 
 #include "../../include/wwcuda.h"
 #include "ww_arith.cuh"
+#include "ww_ladder_case.cuh"
 #include "ww_tests.cuh"
 
 using namespace ww;
@@ -142,8 +143,9 @@ __global__ void k_pipe(int iters, u32 seed, u32 *sink) {
     if (acc == 0x7fffffffu) sink[threadIdx.x] = acc;  // keeps the chains live
 }
 
-// One operation of the device arithmetic per case (the instruction sequences
-// the kernels run), for checking it operand by operand: ops 0-2 as
+// One operation of the canonical device arithmetic per case (what starts and
+// ends the ladders, and the forms they are tested against), for checking it
+// operand by operand: ops 0-2 as
 // ww_selftest_m2, 3 X+Y, 4 X-Y, 5 2X (mod p^2), 6 x0*y0/2^64, 7 x0+y0,
 // 8 (x1:x0)/2^64 (mod p).
 __global__ void k_m2_cases(int op, u64 p, const u64 *xy, u64 n, u64 *out) {
@@ -167,6 +169,32 @@ __global__ void k_m2_cases(int op, u64 p, const u64 *xy, u64 n, u64 *out) {
         out[2 * i] = z.d0;
         out[2 * i + 1] = z.d1;
     }
+}
+
+// The same for the ladders' own operations (ladder_case).
+__global__ void k_ladder_cases(int op, u64 p, const u64 *in, u64 n, u64 *out) {
+    const LzMod m = lz_mod(p, inv64(p));
+    for (u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (u64)gridDim.x * blockDim.x)
+        ladder_case(op, m, in + 6 * i, out + 3 * i);
+}
+
+// Runs launch(in, out) on device copies of n cases of in_words and out_words.
+template <class F>
+int run_cases(int device, const uint64_t *in, uint64_t *out, uint64_t n, int in_words, int out_words, F &&launch) {
+    if (n == 0) return WW_OK;
+    if (cudaSetDevice(device) != cudaSuccess) return WW_ERR_NODEV;
+    u64 *d = nullptr;
+    if (cudaMalloc(&d, n * 8 * (u64)(in_words + out_words)) != cudaSuccess) return WW_ERR_NOMEM;
+    int rc = WW_OK;
+    if (cudaMemcpy(d, in, n * 8 * (u64)in_words, cudaMemcpyHostToDevice) != cudaSuccess) rc = WW_ERR_CUDA;
+    if (rc == WW_OK) {
+        launch((unsigned)((n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184), d, d + n * (u64)in_words);
+        if (cudaGetLastError() != cudaSuccess ||
+            cudaMemcpy(out, d + n * (u64)in_words, n * 8 * (u64)out_words, cudaMemcpyDeviceToHost) != cudaSuccess)
+            rc = WW_ERR_CUDA;
+    }
+    cudaFree(d);
+    return rc;
 }
 
 }  // namespace
@@ -210,21 +238,16 @@ int ww_random_primes(int device, uint64_t seed, uint64_t n, uint64_t *out, uint6
 
 int ww_devtest_m2(int device, int op, uint64_t p, const uint64_t *xy, uint64_t n, uint64_t *out) {
     if ((p & 1) == 0 || p < 3 || ((!xy || !out) && n) || op < 0 || op > 8) return WW_ERR_ARG;
-    if (n == 0) return WW_OK;
-    if (cudaSetDevice(device) != cudaSuccess) return WW_ERR_NODEV;
-    u64 *d = nullptr;
-    if (cudaMalloc(&d, n * 48) != cudaSuccess) return WW_ERR_NOMEM;
-    int rc = WW_OK;
-    if (cudaMemcpy(d, xy, n * 32, cudaMemcpyHostToDevice) != cudaSuccess) rc = WW_ERR_CUDA;
-    if (rc == WW_OK) {
-        const u64 blocks = (n + 255) / 256 < 1184 ? (n + 255) / 256 : 1184;
-        k_m2_cases<<<(unsigned)blocks, 256>>>(op, p, d, n, d + 4 * n);
-        if (cudaGetLastError() != cudaSuccess ||
-            cudaMemcpy(out, d + 4 * n, n * 16, cudaMemcpyDeviceToHost) != cudaSuccess)
-            rc = WW_ERR_CUDA;
-    }
-    cudaFree(d);
-    return rc;
+    return run_cases(device, xy, out, n, 4, 2, [&](unsigned blocks, const u64 *in, u64 *res) {
+        k_m2_cases<<<blocks, 256>>>(op, p, in, n, res);
+    });
+}
+
+int ww_devtest_ladder(int device, int op, uint64_t p, const uint64_t *in, uint64_t n, uint64_t *out) {
+    if ((p & 1) == 0 || p < 3 || ((!in || !out) && n) || op < 0 || op >= kLadderOps) return WW_ERR_ARG;
+    return run_cases(device, in, out, n, 6, 3, [&](unsigned blocks, const u64 *from, u64 *res) {
+        k_ladder_cases<<<blocks, 256>>>(op, p, from, n, res);
+    });
 }
 
 int ww_pipe_bench(int device, int mode, double *ops_per_s, double *ms_out) {

@@ -168,6 +168,8 @@ _SIGS = {
     "ww_batch_run_noalloc": (C.c_int, [C.POINTER(Unit), C.c_uint32, _VP, _VP, _VP, C.c_uint32, _VP, _VP]),
     "ww_selftest_m2": (C.c_int, [C.c_int, C.c_uint64, _U64P, C.c_uint64, _U64P]),
     "ww_devtest_m2": (C.c_int, [C.c_int, C.c_int, C.c_uint64, _U64P, C.c_uint64, _U64P]),
+    "ww_selftest_ladder": (C.c_int, [C.c_int, C.c_uint64, _U64P, C.c_uint64, _U64P]),
+    "ww_devtest_ladder": (C.c_int, [C.c_int, C.c_int, C.c_uint64, _U64P, C.c_uint64, _U64P]),
     "ww_selftest_candidates": (C.c_int, [C.c_uint64, C.c_uint64, _U64P, C.c_uint64, C.POINTER(C.c_uint64),
                                          C.POINTER(C.c_uint64)]),
     "ww_random_primes": (C.c_int, [C.c_int, C.c_uint64, C.c_uint64, _U64P, C.POINTER(C.c_uint64)]),
@@ -273,6 +275,23 @@ def devtest_m2(op: int, p: int, xy: np.ndarray, device: int = 0) -> np.ndarray:
     out = np.zeros(2 * n, dtype=np.uint64)
     check(_L.ww_devtest_m2(device, op, p, xy, n, out), "ww_devtest_m2")
     return out.reshape(-1, 2)
+
+
+def _ladder_cases(name: str, *args) -> np.ndarray:
+    *args, cases = args
+    cases = np.ascontiguousarray(cases, dtype=np.uint64).reshape(-1)
+    n = cases.size // 6
+    out = np.zeros(3 * n, dtype=np.uint64)
+    check(getattr(_L, name)(*args, cases, n, out), name)
+    return out.reshape(-1, 3)
+
+
+def selftest_ladder(op: int, p: int, cases: np.ndarray) -> np.ndarray:
+    return _ladder_cases("ww_selftest_ladder", op, p, cases)
+
+
+def devtest_ladder(op: int, p: int, cases: np.ndarray, device: int = 0) -> np.ndarray:
+    return _ladder_cases("ww_devtest_ladder", device, op, p, cases)
 
 
 def selftest_candidates(lo: int, hi: int) -> tuple[np.ndarray, int]:
