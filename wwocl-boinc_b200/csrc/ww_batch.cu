@@ -182,7 +182,7 @@ int ensure_capacity(BatchState &b, u32 n_units, u32 hit_cap) {
 
 // A finished unit's tiles counted in full ones, whatever they were cut into.
 u32 full_tiles(const UnitState &u, u64 tile) {
-    if (u.tiles_done < u.n_tiles) return (u32)((u64)u.tiles_done * 64 * u.words / tile);
+    if (u.tiles_done < u.n_tiles) return (u32)(u.tiles_done * 64 * u.words / tile);
     const u64 w = u.end - u.start;
     return (u32)(w / tile + (w % tile ? 1 : 0));
 }
@@ -256,7 +256,6 @@ int run_batch(ww_ctx *ctx, BatchState &b, const ww_unit *units, uint32_t n, cons
         const u64 w = units[i].end - units[i].start, tile = 64ull * u.words;
         left -= (double)w;
         u.n_tiles = w / tile + (w % tile ? 1 : 0);
-        u.active = 1;
         b.h_first[i] = acc;
         acc += u.n_tiles;
     }
@@ -735,7 +734,6 @@ int ww_server_step(ww_ctx *ctx, ww_request_result *done, uint32_t cap, uint32_t 
         u.words = std::min(tile_words(left, s.grid, (u32)s.e->seg_words), kServeMaxWords);
         const u64 tile = 64ull * u.words;
         u.n_tiles = w / tile + (w % tile ? 1 : 0);
-        u.active = 1;
         if (s.cfg.store_prps) {
             u.prp_out = s.pool + off / 8;
             u.prp_cap = bound;

@@ -34,8 +34,8 @@ struct UnitState {
     u64 *prp_out;            // optional PRP buffer of the range (nullptr: none)
     u64 prp_cap;
     u64 prp_written;         // PRPs found (may exceed prp_cap: overflow)
-    u32 hits, tiles_done;
-    u32 active;
+    u64 tiles_done;          // 64 bits: tiles of 2^18 numbers in a request of 2^50 pass 2^32
+    u32 hits;
     u32 words;               // bitmap words of a tile of this unit
 };
 
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) k_tiles(BatchA
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();
-            atomicAdd(&a.units[unit].tiles_done, 1u);
+            atomicAdd((unsigned long long *)&a.units[unit].tiles_done, 1ull);
         }
     }
     if (pn > 0) test_batch<Cfg::kPpt, Cfg::kJoint>(pq, uq, pn, a);

@@ -163,7 +163,6 @@ extern "C" int ww_batch_run_noalloc(const ww_unit *units, uint32_t n, ww_unit_re
         const u64 w = units[i].end - units[i].start, tile = 64ull * u.words;
         left -= (double)w;
         u.n_tiles = w / tile + (w % tile ? 1 : 0);
-        u.active = 1;
         g_h_first[i] = acc;
         acc += u.n_tiles;
     }
