@@ -148,6 +148,33 @@ def test_gpu_cut_tiles_equal_units_alone(ww, widths, cfg):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("widths", [[1], [2**13 - 1, 2**13 + 1], [100_000], [300_001] * 5, [40_000_000, 999, 1_000_000],
+                                    [50_000] * 300, [2**28 + 5, 7, 2**20]])
+def test_gpu_cut_tiles_through_the_allocation_free_entry(ww, widths):
+    """The same widths through ww_batch_run_noalloc: the batch's results in
+    its configuration, and the finished tiles counted in full ones."""
+    import ctypes as C
+
+    import torch
+
+    rng = random.Random(len(widths))
+    units = [(a, a + w) for a, w in ((rng.randrange(127, 2**64 - 2**29), w) for w in widths)]
+    with ww.Context(0, max_prps=1 << 12) as ctx:
+        batch = ww.Batch(ctx)
+        batch.set_config(8192, 256, 1)
+        want = [(r["checksum"], r["prp_count"], r["hits"], r["tiles_done"]) for r in batch.run(units)]
+    arr = (ww.Unit * len(units))()
+    for i, (a, b) in enumerate(units):
+        arr[i].start, arr[i].end = a, b
+    out = torch.zeros(len(units) * C.sizeof(ww.UnitResult), dtype=torch.uint8, device="cuda")
+    count = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ww.check(ww.lib().ww_batch_run_noalloc(arr, len(units), out.data_ptr(), None, None, 0, count.data_ptr(),
+                                           torch.cuda.current_stream().cuda_stream), "ww_batch_run_noalloc")
+    got = (ww.UnitResult * len(units)).from_buffer_copy(out.cpu().numpy().tobytes())
+    assert [(r.checksum, r.prp_count, r.hits, r.tiles_done) for r in got] == want
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("cfg", [(16384, 512, 1, 1), (8192, 256, 1, 1)])
 @pytest.mark.parametrize("low", [127, 2**32 - 300_000, 2**32 + 1])
 def test_gpu_joint_loop_around_one_word_primes(ww, cfg, low):

@@ -180,13 +180,6 @@ int ensure_capacity(BatchState &b, u32 n_units, u32 hit_cap) {
     return WW_OK;
 }
 
-// A finished unit's tiles counted in full ones, whatever they were cut into.
-u32 full_tiles(const UnitState &u, u64 tile) {
-    if (u.tiles_done < u.n_tiles) return (u32)(u.tiles_done * 64 * u.words / tile);
-    const u64 w = u.end - u.start;
-    return (u32)(w / tile + (w % tile ? 1 : 0));
-}
-
 void fill_deep_n(BatchArgs &a) {
     for (int k = 0; k < kTileSizes; ++k) a.deep_n[k] = deep_rows_for(64.0 * (kTileMinWords << k), ~0ull);
 }

@@ -39,6 +39,14 @@ struct UnitState {
     u32 words;               // bitmap words of a tile of this unit
 };
 
+// A unit's finished tiles counted in full ones of `tile` numbers, whatever
+// they were cut into.
+WW_HD u32 full_tiles(const UnitState &u, u64 tile) {
+    if (u.tiles_done < u.n_tiles) return (u32)(u.tiles_done * 64 * u.words / tile);
+    const u64 w = u.end - u.start;
+    return (u32)(w / tile + (w % tile ? 1 : 0));
+}
+
 // Tiles have kTileMinWords << k words, k < kTileSizes.
 constexpr int kTileMinWords = 128;
 constexpr int kTileSizes = 9;
@@ -365,6 +373,8 @@ __global__ void __launch_bounds__(Cfg::kThreads, Cfg::kMinBlocks) k_tiles(BatchA
             if (!more) break;
         }
         __syncthreads();
+        // some of the tile's PRPs may still wait in the warps' queues: the
+        // count is read only after the launch, which empties them
         if (threadIdx.x == 0) {
             __threadfence();
             atomicAdd((unsigned long long *)&a.units[unit].tiles_done, 1ull);

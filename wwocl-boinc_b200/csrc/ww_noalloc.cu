@@ -80,8 +80,7 @@ __global__ void k_noalloc_finish(const NoAllocScratch *s, uint32_t n, ww_unit_re
         out[i].checksum = s->units[i].checksum;
         out[i].prp_count = s->units[i].prp_count;
         out[i].hits = s->units[i].hits;
-        const u64 w = s->units[i].end - s->units[i].start;  // every tile is done: counted in full ones
-        out[i].tiles_done = (uint32_t)(w / NoAllocCfg::kTileNumbers + (w % NoAllocCfg::kTileNumbers ? 1 : 0));
+        out[i].tiles_done = full_tiles(s->units[i], NoAllocCfg::kTileNumbers);
     }
     const uint32_t nh = s->hit_count < kNoAllocMaxHits ? s->hit_count : kNoAllocMaxHits;
     for (uint32_t i = tid; i < nh && i < hit_cap; i += gridDim.x * blockDim.x) {
