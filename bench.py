@@ -647,13 +647,14 @@ def main():
                 "ops_per_prime": per_prime,
                 "ops_source": "reference kernels' algorithm: 40(k-3) + 128(k-1) 32-bit multiplies per prime",
                 "frac_note": "frac counts the reference algorithm's multiplies, more than this kernel executes, so "
-                             "it can pass 1.0; executed.frac is the pipe-occupancy view",
+                             "it can pass 1.0; executed.frac counts this kernel's, a 64x64 product as 8 like the "
+                             "chain, though it runs most as four wide ones: the pipe's occupancy is the profile's",
                 "executed": {"ops_per_prime": per_prime_run, "achieved": achieved_run / 1e12,
                              "frac": achieved_run / chain_peak,
                              "note": "multiplies k_test_prps itself runs: 126(k-6) + 134 (ladders started from their top bits, three-product squares of the low digit)"},
                 "mad_lo_only": {"peak": madlo_peak / 1e12, "frac": achieved / madlo_peak,
                                 "frac_executed": achieved_run / madlo_peak},
-                "hbm": {"bytes_per_launch": 16 * n, "GBps": 16 * n / (launch_ms * 1e-3) / 1e9,
+                "hbm": {"bytes_per_launch": 32 * n, "GBps": 32 * n / (launch_ms * 1e-3) / 1e9,  # each test reads p and p^-1
                         "peak_GBps": json.loads(PEAKS.read_text())["hbm_gbs"] if PEAKS.exists() else 6650.0,
                         "peak_source": "measured copy bandwidth" if PEAKS.exists()
                         else "fallback 6.65 TB/s (no measured peaks file)"}}

@@ -179,8 +179,10 @@ int ww_selftest_deep_table(ww_ctx *ctx, int bits, uint64_t first, uint64_t n, ui
  * with the depth, what the program's autotune picks in place of the
  * reference's work-size profiling, main.cpp:959-1107): 1 = segments of 2^20
  * numbers for 512-thread CTAs, 2 = 2^19 numbers for 256-thread CTAs, 0 (the
- * default) = the wide shape when the launch gives each resident CTA a
- * segment, else the narrow one.  Results do not depend on the shape. */
+ * default) = by the launch's width: the wide shape when each resident CTA
+ * gets two of its segments (6.2e8 numbers on a B200), below that segments of
+ * 2^11 to 2^19 numbers for 256-thread CTAs, cut so that every resident CTA
+ * gets the same number of them.  Results do not depend on the shape. */
 int ww_set_sieve_shape(ww_ctx *ctx, int shape);
 int ww_get_sieve_shape(ww_ctx *ctx, int *shape);
 int ww_wieferich(ww_ctx *ctx);

@@ -251,10 +251,10 @@ WW_HD u64 r_mod(u64 n) {
     return (0 - n) % n;
 }
 
-// T mod n and floor(T / n) for T = h 2^64 + l < 2^48 n, n odd and > 1, with
-// rn = 1.0 / (double)n.  The quotient (below 2^48) is estimated in double
+// T mod n and floor(T / n) for T = h 2^64 + l < 2^50 n, n odd and > 1, with
+// rn = 1.0 / (double)n.  The quotient (below 2^50) is estimated in double
 // precision: T and rn each carry a relative rounding error of at most 2^-52
-// and the product one more rounding, so the estimate is within 2^-2 of T / n
+// and the product one more rounding, so the estimate is within 5/8 of T / n
 // and its truncation is the quotient or one off it; T - qe n then lies in
 // [-n, 2n) and one exact correction finishes.  Host and device run the same
 // steps.  This is how the ladders start from their top bits (a small power
@@ -543,9 +543,9 @@ WW_HD D2 m2_one(u64 p) {
     return r;
 }
 
-// L R mod p^2 as canonical digits for L < 2^48 - 1, from the Montgomery one
+// L R mod p^2 as canonical digits for L <= 2^48, from the Montgomery one
 // (R mod p^2 = o0 + p o1): L o0 = d0 + p q0 with d0 < p, then d1 = (q0 + L o1)
-// mod p.  Both reductions see a number below 2^48 p (mod_est); rp = 1/(double)p.
+// mod p.  Both reductions see a number of at most 2^48 p (mod_est); rp = 1/(double)p.
 WW_HD D2 m2_small(u64 L, D2 one, u64 p, double rp) {
     u64 l, h, q0, q1;
     D2 r;

@@ -93,9 +93,8 @@ struct BatchCfg {
     // 32 warps) with one or two batches of PRPs per warp -- left to the
     // compiler, the 512-thread tiles took 128 registers (16 warps per SM)
     // and ran 7 % slower; four or eight batches keep the compiler's choice
-    // (142 and 146 registers at 256 threads), which measured faster than
-    // 78 and 80 registers at three CTAs per SM (they spill 128 and 256 bytes
-    // at 64)
+    // (110 registers at 256 threads, two CTAs per SM; 142 and 146 while the
+    // batches were written out, then faster than 78 and 80 at three CTAs)
     static constexpr int kSmThreads = PPT >= 4 ? THREADS : 1024;
     static constexpr int kMinBlocks = kSmThreads / THREADS > 0 ? kSmThreads / THREADS : 1;
     static constexpr u64 kTileNumbers = 64ull * SEG_WORDS;  // integers per full tile

@@ -408,7 +408,11 @@ int launch_sieve(uint64_t low, uint64_t high, int32_t wheelidx, uint64_t *g_prim
         const u64 b = high - a > kLargeMarksPiece ? a + kLargeMarksPiece : high;
         const u64 lo = a == b0 ? low : a;  // pieces after the first start on an even number
         const u64 nodd = (b - a) / 2;
-        // whole segments of the wide shape (2^19 odd numbers) cover either shape's reads
+        // zeroed and marked up to a whole segment of the wide shape (2^19 odd
+        // numbers).  The small shape's last segment may read up to 8191 words
+        // past that, from earlier launches: still inside the bitmap (it takes
+        // pieces below 6.2e8 numbers, the bitmap has room for 2^30), and words
+        // past the last odd number are masked in the segment
         const u64 words = ((nodd + SieveWide::kOdd - 1) / SieveWide::kOdd) * (u64)SieveWide::kWords;
         if (words > large->words) return set_err("mark bitmap too small"), WW_ERR_STATE;
         // a narrow piece takes the table's smaller primes only, below 0.4 of

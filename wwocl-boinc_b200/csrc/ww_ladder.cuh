@@ -380,8 +380,9 @@ WW_HD D2 lz_shift(D2 x, u32 d, const LzMod &m) {
 // 0 <= d < 32 (one-word Montgomery steps: 6 instructions a bit for two digits
 // where a conditional doubling takes 18, 3 against 11 for one).  With
 // f = e + sum of 32^(w+1) over the windows w, e is the start f >> steps
-// (below 48 where e >> steps is below 32) times 2^steps plus the sum of
-// (d_w - 32) 32^w.
+// times 2^steps plus the sum of (d_w - 32) 32^w.  Where e >> steps is below
+// 32 the start is at most 48 (steps = 5 w + 1 and an exponent of ones: 31,
+// 16 from the top window's 32^w and a carry).
 constexpr int kWinBits = 5;
 WW_HD u64 power_windows(u64 e, int steps) {
     // 32 + 32^2 + ... for ceil(steps / 5) windows

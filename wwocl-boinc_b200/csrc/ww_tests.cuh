@@ -117,11 +117,11 @@ WW_HD int ladder_steps(u64 j) {
     return top > 4 ? top - 4 : 0;
 }
 
-// L R mod p^2 as canonical digits for L < 2^48.  For p >= 2^62 the quotient
-// of L 2^64 by p is below 2^50 and mod_est's estimate within 2^-1 of it (three
-// roundings of 2^-53 and those of (double)p), so its correction by one is
-// still enough; and it is the high digit as it stands: one reduction, where
-// m2_small needs two and the products with the digits of R.
+// L R mod p^2 as canonical digits for L <= 2^48 (a power of 2 of the Wieferich
+// start; Lucas numbers are below 2^46), below 2^48 for p >= 2^62.  There the
+// quotient of L 2^64 by p is below 2^50, as mod_est wants it, and it is the
+// high digit as it stands: one reduction, where m2_small needs two and the
+// products with the digits of R.
 WW_HD D2 small_start(u64 L, D2 one, u64 p, double rp) {
     if (p >> 62) {
         D2 r;
@@ -200,7 +200,7 @@ WW_HD SmallMod small_mod(u64 p) {
     s.rn = 1.0 / (double)n;
     return s;
 }
-// L R mod n for 1 <= L < 2^48
+// L R mod n for 1 <= L <= 2^48
 WW_HD u64 small_times_r(u64 L, const SmallMod &s) {
     u64 l, h, unused;
     mul_wide(L, s.one, l, h);
